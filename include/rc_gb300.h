@@ -306,8 +306,10 @@ int gb_gcf_generate(int32_t n_planes, const double *w_planes, const int32_t *sup
  * (psf_peak_x, psf_peak_y) lands on the residual peak (zero outside the PSF);
  * model[peak] += gain * peak.  Images are row-major nx * ny floats; the PSF
  * pnx * pny.  d_work: gb_hogbom_work_bytes() bytes of device scratch.  One
- * launch per iteration, no synchronisation: the sequence can be captured in
- * a CUDA graph.  gb_hogbom_iterations reads back how many iterations
+ * cooperative launch of at most one CTA per SM, no synchronisation: it can be
+ * captured in a CUDA graph.  The CTAs wait for one another with a bound; if a
+ * wait ever ran out, the images are invalid and gb_hogbom_iterations returns
+ * GB_ERR_TIMEOUT.  gb_hogbom_iterations reads back how many iterations
  * subtracted a component (synchronises). */
 int gb_hogbom_work_bytes(int32_t nx, int32_t ny, int64_t *bytes);
 int gb_hogbom_f32(float *d_residual, int32_t nx, int32_t ny, const float *d_psf, int32_t pnx,
