@@ -13,7 +13,8 @@
 //
 // FFT is exp(-2 pi i) (cuFFT forward), IFFT_unnorm exp(+2 pi i) without the
 // 1/N^2, so A^H is the adjoint of A for the real inner product on images.
-// For even N, fftshift and ifftshift are the same permutation.
+// For even N, fftshift and ifftshift are the same permutation.  FP32 sizes with
+// small prime factors take the fused passes of gb_fft.cu instead.
 #include <cufft.h>
 
 #include <map>
@@ -21,6 +22,7 @@
 #include <tuple>
 
 #include "gb_common.cuh"
+#include "gb_fft.cuh"
 #include "rc_gb300_ms5.h"
 #include "gb_runtime.cuh"
 
@@ -158,6 +160,8 @@ static int image_to_grid(const R* x, const R* t, int n, typename Cx<R>::T* g, cu
     gb_set_error(GB_ERR_ARG, "image_to_grid: NULL buffer or odd/too small n=%d", n);
     return GB_ERR_ARG;
   }
+  if constexpr (sizeof(R) == 4)
+    if (fft_size_ok(n)) return fft_image_to_grid(x, t, n, g, s);
   const int64_t nn = (int64_t)n * n;
   k_image_in<R><<<blocks_nn(nn), 256, 0, s>>>(x, t, n, g);
   GB_CUDA_TRY(cudaGetLastError());
@@ -175,6 +179,8 @@ static int grid_to_image(const typename Cx<R>::T* g, const R* t, int n, typename
     gb_set_error(GB_ERR_ARG, "grid_to_image: NULL/aliased buffer or odd/too small n=%d", n);
     return GB_ERR_ARG;
   }
+  if constexpr (sizeof(R) == 4)
+    if (fft_size_ok(n)) return fft_grid_to_image(g, t, n, w, x, s);
   const int64_t nn = (int64_t)n * n;
   k_shift_copy<<<blocks_nn(nn), 256, 0, s>>>(g, n, w);
   GB_CUDA_TRY(cudaGetLastError());
