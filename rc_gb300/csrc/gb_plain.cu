@@ -118,8 +118,14 @@ __global__ void k_max_exponent(const double* __restrict__ x, int64_t rows, int64
       m = max(m, e == 0 && (b & 0xFFFFFFFFFFFFFull) ? kExpNonFinite : e);
     }
   }
+  // one atomic per block, and none where it changes nothing
+  __shared__ int s_m;
+  if (threadIdx.x == 0) s_m = 0;
+  __syncthreads();
   m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_m, m);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_m > *(volatile int*)out) atomicMax(out, s_m);
 }
 
 // The scale exponent of an array from its largest exponent field: the array
@@ -314,26 +320,6 @@ __device__ __forceinline__ LaneIndex single_index(const double* __restrict__ vis
 __device__ __forceinline__ int64_t visit_rec(const int32_t* __restrict__ order, int64_t i,
                                              int64_t n) {
   return order && i < n ? (int64_t)order[i] : i;
-}
-
-__global__ void k_scatter_single64(int64_t n, const double* __restrict__ vis5,
-                                   const double2* __restrict__ gcf, double2* __restrict__ grid,
-                                   SingleGeo geo, const int32_t* __restrict__ order) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t t0 = 32 * (blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5)); t0 < n;
-       t0 += 32 * warps) {
-    const int64_t t = visit_rec(order, t0 + lane, n);
-    const LaneIndex mine = single_index(vis5, t, n, geo);
-    const int m = (int)min((int64_t)32, n - t0);
-    for (int j = 0; j < m; j++) {
-      const LaneIndex ix = mine.from(j);
-      if (!ix.keep) continue;
-      const double* r = vis5 + 5 * __shfl_sync(0xffffffffu, t, j);
-      warp_scatter64(grid + (int64_t)ix.y0 * geo.pitch + ix.x0, geo.pitch,
-                     gcf + (int64_t)ix.phase * geo.S * geo.S, geo.S, r[3], r[4], lane);
-    }
-  }
 }
 
 // vis_out = vis; in-bound: vis_out.re/im -= sum grid * gcf (degrid.cpp:78-98).
@@ -543,19 +529,58 @@ __global__ void k_add_c128(double2* __restrict__ a, const double2* __restrict__ 
 // whole grid is copied as before (host_direct, gb_runtime.cu).
 constexpr int kBlk = 32;
 
-// marks[by * nbx + bx] = 1 for every block a kept footprint overlaps
-__global__ void k_mark_blocks(int64_t n, const double* __restrict__ vis5, SingleGeo geo, int nbx,
-                              unsigned char* __restrict__ marks) {
+// One pass over a call's records: the block (key) of each one's footprint
+// corner (nkeys - 1 for a record that is not kept) and how many records each
+// key has; with `marks`, marks[by * nbx + bx] = 1 for every block a kept
+// footprint overlaps; with `exp`, *exp max-ed with the largest exponent field of
+// the visibilities (k_max_exponent's rule).  A warp's records mostly share a
+// few keys (neighbouring samples of a baseline): one atomic per key and warp.
+// On 100,000 records over a 1024^2 grid this takes 23 to 41 us and the scatter
+// below 7 us; with marks, exponent, histogram and scatter as kernels of their own,
+// an atomic per record or warp, they took 15, 129, 35 and 33 us.
+__global__ void __launch_bounds__(256) k_record_keys(int64_t n, const double* __restrict__ vis5,
+                                                     SingleGeo geo, int nbx, int nkeys,
+                                                     unsigned char* __restrict__ marks,
+                                                     int32_t* __restrict__ keys,
+                                                     int32_t* __restrict__ hist,
+                                                     int* __restrict__ exp) {
+  int m = 0;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const VisIndex ix = vis_index(vis5[5 * t], vis5[5 * t + 1], geo.scale, geo.grid_size, geo.S,
-                                  geo.margin, geo.min_x, geo.min_y, geo.ext_x, geo.ext_y);
-    if (!ix.keep) continue;
-    const int x0 = ix.x0 - geo.min_x, y0 = ix.y0 - geo.min_y;
-    const int bx1 = (x0 + geo.S - 1) / kBlk, by1 = (y0 + geo.S - 1) / kBlk;
-    for (int by = y0 / kBlk; by <= by1; by++)
-      for (int bx = x0 / kBlk; bx <= bx1; bx++) marks[by * nbx + bx] = 1;
+    const double* r = vis5 + 5 * t;
+    const VisIndex ix = vis_index(r[0], r[1], geo.scale, geo.grid_size, geo.S, geo.margin,
+                                  geo.min_x, geo.min_y, geo.ext_x, geo.ext_y);
+    int key = nkeys - 1;
+    if (ix.keep) {
+      const int x0 = ix.x0 - geo.min_x, y0 = ix.y0 - geo.min_y;
+      key = (y0 / kBlk) * nbx + x0 / kBlk;
+      if (marks) {
+        const int bx1 = (x0 + geo.S - 1) / kBlk, by1 = (y0 + geo.S - 1) / kBlk;
+        for (int by = y0 / kBlk; by <= by1; by++)
+          for (int bx = x0 / kBlk; bx <= bx1; bx++)
+            if (!marks[by * nbx + bx]) marks[by * nbx + bx] = 1;
+      }
+    }
+    keys[t] = key;
+    const unsigned act = __activemask(), peers = __match_any_sync(act, key);
+    if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&hist[key], __popc(peers));
+    if (exp) {
+#pragma unroll
+      for (int h = 3; h < 5; h++) {
+        const unsigned long long b = (unsigned long long)__double_as_longlong(r[h]);
+        const int e = (int)((b >> 52) & 0x7FF);
+        m = max(m, e == 0 && (b & 0xFFFFFFFFFFFFFull) ? kExpNonFinite : e);
+      }
+    }
   }
+  if (!exp) return;
+  __shared__ int s_m;
+  if (threadIdx.x == 0) s_m = 0;
+  __syncthreads();
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_m, m);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_m) atomicMax(exp, s_m);
 }
 
 // One CTA per block of a W x H complex128 region (device rows W apart):
@@ -613,7 +638,7 @@ __global__ void k_gather_host(double2* __restrict__ d, const double* __restrict_
     }
   }
   m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(exp, m);
+  if ((threadIdx.x & 31) == 0 && m > *(volatile int*)exp) atomicMax(exp, m);
 }
 
 // The double-float split of d (W x H, rows W apart) on the marked blocks,
@@ -634,33 +659,6 @@ __global__ void k_df_split_marked(const double2* __restrict__ d, int W, int H, i
       out[(int64_t)y * W + x] = make_float4(re.x, re.y, im.x, im.y);
     }
   }
-}
-
-// Marks of the kept footprints of n device records over a W x H region.
-static int mark_blocks(int64_t n, const void* d_vis, const SingleGeo& geo, int nbx, int nby,
-                       unsigned char* marks, cudaStream_t s) {
-  GB_CUDA_TRY(cudaMemsetAsync(marks, 0, (size_t)nbx * nby, s));
-  const int blocks = (int)std::clamp<int64_t>((n + 255) / 256, 1, (int64_t)sm_count() * 8);
-  k_mark_blocks<<<blocks, 256, 0, s>>>(n, (const double*)d_vis, geo, nbx, marks);
-  GB_CUDA_TRY(cudaGetLastError());
-  return GB_OK;
-}
-
-// Counting sort of a call's records by the kBlk x kBlk block of their
-// footprint corner (kept records; the others last), on the device: a
-// histogram, a one-block exclusive scan, a scatter of record indices.
-__device__ __forceinline__ int block_key(const double* __restrict__ vis5, int64_t t,
-                                         const SingleGeo& geo, int nbx, int nkeys) {
-  const VisIndex ix = vis_index(vis5[5 * t], vis5[5 * t + 1], geo.scale, geo.grid_size, geo.S,
-                                geo.margin, geo.min_x, geo.min_y, geo.ext_x, geo.ext_y);
-  return ix.keep ? ((ix.y0 - geo.min_y) / kBlk) * nbx + (ix.x0 - geo.min_x) / kBlk : nkeys - 1;
-}
-
-__global__ void k_key_hist(int64_t n, const double* __restrict__ vis5, SingleGeo geo, int nbx,
-                           int nkeys, int32_t* __restrict__ hist) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
-       t += (int64_t)gridDim.x * blockDim.x)
-    atomicAdd(&hist[block_key(vis5, t, geo, nbx, nkeys)], 1);
 }
 
 // offs = exclusive scan of hist over nkeys entries (one block of 1024 threads)
@@ -686,36 +684,45 @@ __global__ void __launch_bounds__(1024) k_scan_keys(const int32_t* __restrict__ 
   }
 }
 
-__global__ void k_key_scatter(int64_t n, const double* __restrict__ vis5, SingleGeo geo, int nbx,
-                              int nkeys, const int32_t* __restrict__ offs,
-                              int32_t* __restrict__ cursor, int32_t* __restrict__ order) {
+__global__ void k_key_scatter(int64_t n, const int32_t* __restrict__ keys,
+                              const int32_t* __restrict__ offs, int32_t* __restrict__ cursor,
+                              int32_t* __restrict__ order) {
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int k = block_key(vis5, t, geo, nbx, nkeys);
-    order[offs[k] + atomicAdd(&cursor[k], 1)] = (int32_t)t;
+    const int k = keys[t], lane = threadIdx.x & 31;
+    const unsigned act = __activemask(), peers = __match_any_sync(act, k);
+    const int leader = __ffs(peers) - 1;
+    int first = 0;
+    if (lane == leader) first = atomicAdd(&cursor[k], __popc(peers));
+    first = __shfl_sync(act, first, leader);
+    order[offs[k] + first + __popc(peers & ((1u << lane) - 1u))] = (int32_t)t;
   }
 }
 
-// The visit order of n device records (staging slots 7 and 8).
-static int order_by_block(int64_t n, const void* d_vis, const SingleGeo& geo, int32_t** order,
-                          cudaStream_t s) {
+// The visit order of n device records: a counting sort by the kBlk x kBlk block
+// of their footprint corner (kept records; the others last).  With `marks` (one
+// byte per block) the blocks that kept footprints touch, with `exp` (zeroed by
+// the caller) the visibilities' largest exponent field.  Staging slots 7 and 8.
+static int prepare_records(int64_t n, const void* d_vis, const SingleGeo& geo,
+                           unsigned char* marks, int* exp, int32_t** order, cudaStream_t s) {
   const int nbx = (geo.ext_x + kBlk - 1) / kBlk, nby = (geo.ext_y + kBlk - 1) / kBlk;
   const int nkeys = nbx * nby + 1;
   void *d_keys, *d_order;
   int rc;
   if ((rc = stage_buffer(7, (size_t)3 * nkeys * sizeof(int32_t), &d_keys)) ||
-      (rc = stage_buffer(8, (size_t)n * sizeof(int32_t), &d_order)))
+      (rc = stage_buffer(8, (size_t)2 * n * sizeof(int32_t), &d_order)))
     return rc;
   int32_t* hist = (int32_t*)d_keys;
   int32_t* offs = hist + nkeys;
   int32_t* cursor = offs + nkeys;
-  GB_CUDA_TRY(cudaMemsetAsync(hist, 0, sizeof(int32_t) * nkeys, s));
-  GB_CUDA_TRY(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * nkeys, s));
+  int32_t* keys = (int32_t*)d_order + n;
+  GB_CUDA_TRY(cudaMemsetAsync(hist, 0, sizeof(int32_t) * 3 * nkeys, s));
+  if (marks) GB_CUDA_TRY(cudaMemsetAsync(marks, 0, (size_t)nbx * nby, s));
   const int blocks = (int)std::clamp<int64_t>((n + 255) / 256, 1, (int64_t)sm_count() * 8);
-  const double* v = (const double*)d_vis;
-  k_key_hist<<<blocks, 256, 0, s>>>(n, v, geo, nbx, nkeys, hist);
+  k_record_keys<<<blocks, 256, 0, s>>>(n, (const double*)d_vis, geo, nbx, nkeys, marks, keys, hist,
+                                       exp);
   k_scan_keys<<<1, 1024, 0, s>>>(hist, offs, nkeys);
-  k_key_scatter<<<blocks, 256, 0, s>>>(n, v, geo, nbx, nkeys, offs, cursor, (int32_t*)d_order);
+  k_key_scatter<<<blocks, 256, 0, s>>>(n, keys, offs, cursor, (int32_t*)d_order);
   GB_CUDA_TRY(cudaGetLastError());
   *order = (int32_t*)d_order;
   return GB_OK;
@@ -728,8 +735,10 @@ static int df_prepare(const double* grid, int32_t ext_x, int32_t ext_y, int64_t 
                       int* exps, cudaStream_t s) {
   GB_CUDA_TRY(cudaMemsetAsync(exps, 0, 2 * sizeof(int), s));
   const int64_t row = 2 * (int64_t)ext_x;
-  const dim3 gg((unsigned)std::clamp<int64_t>((row + 255) / 256, 1, 64),
-                (unsigned)std::clamp<int64_t>(ext_y, 1, 4096));
+  // about 16 blocks per SM over the grid's rows
+  const int64_t gx = std::clamp<int64_t>((row + 255) / 256, 1, 64);
+  const dim3 gg((unsigned)gx, (unsigned)std::clamp<int64_t>((int64_t)sm_count() * 16 / gx, 1,
+                                                            std::max(1, ext_y)));
   const dim3 gc((unsigned)std::clamp<int64_t>((2 * n_gcf + 255) / 256, 1, (int64_t)sm_count() * 4),
                 1);
   k_max_exponent<<<gg, 256, 0, s>>>(grid, ext_y, row, 2 * pitch, exps);
@@ -743,7 +752,7 @@ static int df_prepare(const double* grid, int32_t ext_x, int32_t ext_y, int64_t 
 // ---------------------------------------------------------------- ABI gridding in shared memory
 // kern_scatter_gpu1 and its siblings (every GCF size they accept: 8, 16, 32
 // and 64).  A call's kept records, counting-sorted by the kBlk x kBlk block of
-// their footprint corner (order_by_block), are cut into chunks of up to
+// their footprint corner (prepare_records), are cut into chunks of up to
 // ScatShape<S>::CH consecutive records (fewer for a call with few records),
 // one CTA per chunk.  A CTA accumulates the records of
 // one block at a time in shared memory, over the block's footprint region
@@ -884,42 +893,37 @@ __global__ void __launch_bounds__(ScatShape<S>::NT)
   if (cur >= 0) flush();
 }
 
-// Gridding of a call's n device records into the device grid `grid` (W x H,
-// rows W apart; zero, or zero on the blocks the records touch): the
-// shared-memory double-float kernel for GCF sizes 8, 16, 32 and 64, the warp
-// kernel with FP64 atomics otherwise.  Staging slots 5 (GCF split, exponents),
-// 7 and 8 (the records' order).
+// Scratch of scatter_records (staging slot 5): the GCF's split and, behind it,
+// the exponent words: [0] the visibilities' (fields 3 and 4 of each record),
+// [1] the GCF's, both zeroed here.
+static int scatter_scratch(int S, float4** gcf_df, int** exps, cudaStream_t s) {
+  const int64_t n_gcf = (int64_t)GB_PHASES * S * S;
+  void* d;
+  const int rc = stage_buffer(5, (size_t)n_gcf * 16 + 16, &d);
+  if (rc) return rc;
+  *gcf_df = (float4*)d;
+  *exps = (int*)((char*)d + (size_t)n_gcf * 16);
+  GB_CUDA_TRY(cudaMemsetAsync(*exps, 0, 2 * sizeof(int), s));
+  return GB_OK;
+}
+
+// Gridding of a call's n device records, in the order that prepare_records made
+// (staging slot 7 holds its hist, offs, cursor), into the device grid `grid` (W x
+// H, rows W apart; zero, or zero on the blocks the records touch).
 static int scatter_records(int64_t n, const void* d_vis, const void* d_gcf, double2* grid,
-                           const SingleGeo& geo, const int32_t* order, cudaStream_t s) {
+                           const SingleGeo& geo, const int32_t* order, float4* gcf_df, int* exps,
+                           cudaStream_t s) {
   const int S = geo.S;
   int rc;
-  if (!order && (rc = order_by_block(n, d_vis, geo, (int32_t**)&order, s))) return rc;
-  if (S != 8 && S != 16 && S != 32 && S != 64) {
-    int blocks;
-    const int threads = plain_grid_dims(n, &blocks);
-    k_scatter_single64<<<blocks, threads, 0, s>>>(n, (const double*)d_vis,
-                                                  (const double2*)d_gcf, grid, geo, order);
-    GB_CUDA_TRY(cudaGetLastError());
-    return GB_OK;
-  }
   const int64_t n_gcf = (int64_t)GB_PHASES * S * S;
-  void* d_df;
-  if ((rc = stage_buffer(5, (size_t)n_gcf * 16 + 16, &d_df))) return rc;
-  float4* gcf_df = (float4*)d_df;
-  int* exps = (int*)((char*)d_df + (size_t)n_gcf * 16);
-  // exps[0]: the visibilities' (fields 3 and 4 of each record), exps[1]: the GCF's
-  GB_CUDA_TRY(cudaMemsetAsync(exps, 0, 2 * sizeof(int), s));
-  const int vb = (int)std::clamp<int64_t>((n + 255) / 256, 1, 4096);
   const dim3 gc((unsigned)std::clamp<int64_t>((2 * n_gcf + 255) / 256, 1, (int64_t)sm_count() * 4),
                 1);
-  k_max_exponent<<<dim3(1, vb), 32, 0, s>>>((const double*)d_vis + 3, n, 2, 5, exps);
   k_max_exponent<<<gc, 256, 0, s>>>((const double*)d_gcf, 1, 2 * n_gcf, 2 * n_gcf, exps + 1);
   k_df_split<<<gc, 256, 0, s>>>((const double*)d_gcf, 1, 2 * n_gcf, 2 * n_gcf, exps, 1,
                                 (float2*)gcf_df);
   GB_CUDA_TRY(cudaGetLastError());
   const int nbx = (geo.ext_x + kBlk - 1) / kBlk, nby = (geo.ext_y + kBlk - 1) / kBlk;
   const int nkeys = nbx * nby + 1;
-  // order_by_block keeps (hist, offs, cursor) in slot 7
   void* d_keys;
   if ((rc = stage_buffer(7, (size_t)3 * nkeys * sizeof(int32_t), &d_keys))) return rc;
   const int32_t* offs = (const int32_t*)d_keys + nkeys;
@@ -1113,11 +1117,13 @@ static int compat_scatter(const char* who, int size_err, double scale, int32_t g
     SingleGeo geo{scale, grid_size, margin, S, uvg->min[1], uvg->min[2], W, H, (int64_t)W};
     unsigned char* marks = (unsigned char*)d_marks;
     int32_t* order = nullptr;
-    if ((rc = mark_blocks(n, d_vis, geo, nbx, nby, marks, s)) ||
-        (rc = order_by_block(n, d_vis, geo, &order, s)))
+    float4* gcf_df;
+    int* exps;
+    if ((rc = scatter_scratch(S, &gcf_df, &exps, s)) ||
+        (rc = prepare_records(n, d_vis, geo, marks, exps, &order, s)))
       return rc;
     k_zero_marked<<<nbx * nby, 256, 0, s>>>((double2*)d_acc, W, H, nbx, marks);
-    if ((rc = scatter_records(n, d_vis, d_gcf, (double2*)d_acc, geo, order, s))) {
+    if ((rc = scatter_records(n, d_vis, d_gcf, (double2*)d_acc, geo, order, gcf_df, exps, s))) {
       cudaStreamSynchronize(s);
       return rc;
     }
@@ -1146,7 +1152,12 @@ static int compat_scatter(const char* who, int size_err, double scale, int32_t g
   GB_CUDA_TRY(cudaEventRecord(ev, s));
   GB_CUDA_TRY(cudaStreamWaitEvent(s2, ev, 0));
   SingleGeo geo{scale, grid_size, margin, S, uvg->min[1], uvg->min[2], W, H, (int64_t)W};
-  if ((rc = scatter_records(n, d_vis, d_gcf, (double2*)d_acc, geo, nullptr, s2))) {
+  int32_t* order = nullptr;
+  float4* gcf_df;
+  int* exps;
+  if ((rc = scatter_scratch(S, &gcf_df, &exps, s2)) ||
+      (rc = prepare_records(n, d_vis, geo, nullptr, exps, &order, s2)) ||
+      (rc = scatter_records(n, d_vis, d_gcf, (double2*)d_acc, geo, order, gcf_df, exps, s2))) {
     cudaStreamSynchronize(s);
     cudaStreamSynchronize(s2);
     return rc;
@@ -1210,13 +1221,14 @@ static int compat_degrid(const char* who, int size_err, double scale, int32_t gr
   GB_CUDA_TRY(cudaMemcpyAsync(d_gcf, gcf->host, gcf_bytes, cudaMemcpyHostToDevice, s));
   SingleGeo geo{scale, grid_size, margin, S, uvg->min[1], uvg->min[2], W, H, (int64_t)W};
   const bool direct = host_direct(uvg->host, row);
+  int32_t* order = nullptr;  // of the direct path
   if (direct) {
     // only the blocks the visibilities read, straight from the caller's grid
     void* d_marks;
     const int nbx = (W + kBlk - 1) / kBlk, nby = (H + kBlk - 1) / kBlk;
     if ((rc = stage_buffer(6, (size_t)nbx * nby, &d_marks))) return rc;
     unsigned char* marks = (unsigned char*)d_marks;
-    if ((rc = mark_blocks(n, d_vis, geo, nbx, nby, marks, s))) return rc;
+    if ((rc = prepare_records(n, d_vis, geo, marks, nullptr, &order, s))) return rc;
     // the grid's blocks gathered with their exponent, then split; the GCF's
     // exponent and split as df_prepare makes them
     const int64_t n_gcf = (int64_t)GB_PHASES * S * S;
@@ -1243,8 +1255,6 @@ static int compat_degrid(const char* who, int size_err, double scale, int32_t gr
   if (direct) {
     // one launch over the records in grid-block order (neighbouring warps
     // gather from the same grid lines), then one download of the results
-    int32_t* order = nullptr;
-    if ((rc = order_by_block(n, d_vis, geo, &order, s))) return rc;
     int blocks, pw;
     const int threads = single_degrid_dims(n, &blocks, &pw);
     k_degrid_single64<<<blocks, threads, 0, s>>>(
