@@ -112,6 +112,29 @@ static int build_members(gb_batch* B, int32_t n, const gb_batch_member* m, cudaS
   return GB_OK;
 }
 
+// One member's items on their way into the batch.
+struct alignas(16) MemberItems {
+  const Item* items;
+  const float* cost;
+  int32_t n, first;   // how many, and where they go
+  int64_t rec0;       // the member's first record in the batch
+  int32_t cls[kMaxClasses];  // its classes in the batch's table
+};
+
+// block m: member m's items.
+__global__ void k_merge_items(const MemberItems* __restrict__ members, Item* __restrict__ items,
+                              float* __restrict__ cost, int16_t* __restrict__ grids) {
+  const MemberItems& m = members[blockIdx.x];
+  for (int i = threadIdx.x; i < m.n; i += blockDim.x) {
+    Item it = m.items[i];
+    it.cls = (int16_t)((it.cls & ~kItemClassMask) | m.cls[item_class(it.cls)]);
+    it.start += (int32_t)m.rec0;
+    items[m.first + i] = it;
+    cost[m.first + i] = m.cost[i];
+    grids[m.first + i] = (int16_t)blockIdx.x;
+  }
+}
+
 static int batch_build(gb_batch* B, int32_t n, const gb_batch_member* m, cudaStream_t s) {
   int rc = build_members(B, n, m, s);
   if (rc) return rc;
@@ -162,19 +185,19 @@ static int batch_build(gb_batch* B, int32_t n, const gb_batch_member* m, cudaStr
   for (int st : {0, 2}) B->ctas_degrid[st] = tiled_ctas_per_sm_for(B->NT, false, B->smem_degrid, st);
 
   // merged records and items
-  std::vector<HostItem> items;
-  int64_t off = 0;
+  std::vector<int> counts((size_t)B->n_classes * n, 0);
+  std::vector<MemberItems> mi(n);
+  int64_t off = 0, n_items = 0;
   for (int i = 0; i < n; i++) {
     gb_plan* p = B->members[i];
-    for (HostItem h : p->host_items) {
-      const int u = (int)(std::lower_bound(widths.begin(), widths.end(),
-                                           p->cls[item_class(h.it.cls)].L) -
+    mi[i] = MemberItems{p->d_raw_items, p->d_raw_cost, p->n_items, (int32_t)n_items, off, {}};
+    for (int c = 0; c < p->n_classes; c++) {
+      const int u = (int)(std::lower_bound(widths.begin(), widths.end(), p->cls[c].L) -
                           widths.begin());
-      h.it.cls = (int16_t)((h.it.cls & ~kItemClassMask) | u);
-      h.it.start += (int32_t)off;
-      h.grid = i;
-      items.push_back(h);
+      mi[i].cls[c] = u;
+      counts[(size_t)u * n + i] += p->class_items[c];
     }
+    n_items += p->n_items;
     off += p->n_recs;
     B->kept += p->kept;
     B->taps += p->taps;
@@ -186,11 +209,8 @@ static int batch_build(gb_batch* B, int32_t n, const gb_batch_member* m, cudaStr
     gb_set_error(GB_ERR_CAPACITY, "gb_batch_create: more than 2^31 footprint pieces");
     return GB_ERR_CAPACITY;
   }
-  std::vector<Item> it_out;
-  std::vector<Bundle> b_out;
-  make_bundles(items, B->cls, B->n_classes, it_out, b_out);
-  B->n_items = (int)it_out.size();
-  B->n_bundles = (int)b_out.size();
+  B->n_items = (int)n_items;
+  B->n_bundles = count_bundles(counts, B->cls, n);
   if ((rc = dev_alloc((void**)&B->d_recs, sizeof(Rec) * (B->n_recs ? B->n_recs : 1), "batch")) ||
       (rc = dev_alloc((void**)&B->d_items, sizeof(Item) * (B->n_items ? B->n_items : 1),
                       "batch")) ||
@@ -205,17 +225,35 @@ static int batch_build(gb_batch* B, int32_t n, const gb_batch_member* m, cudaStr
                                   cudaMemcpyDeviceToDevice, s));
     off += p->n_recs;
   }
-  if (B->n_items)
-    GB_CUDA_TRY(cudaMemcpyAsync(B->d_items, it_out.data(), sizeof(Item) * B->n_items,
-                                cudaMemcpyHostToDevice, s));
-  if (B->n_bundles)
-    GB_CUDA_TRY(cudaMemcpyAsync(B->d_bundles, b_out.data(), sizeof(Bundle) * B->n_bundles,
-                                cudaMemcpyHostToDevice, s));
+  // the members' items one after the other, with the batch's classes and record
+  // offsets, then bundled together
+  {
+    unsigned char* d = nullptr;
+    const size_t mb = sizeof(MemberItems) * n;
+    if ((rc = dev_alloc((void**)&d, mb + (sizeof(Item) + sizeof(float) + sizeof(int16_t)) * n_items,
+                        "batch")))
+      return rc;
+    struct Tmp {
+      void* p;
+      ~Tmp() { cudaFree(p); }
+    } tmp{d};
+    static_assert(sizeof(MemberItems) % 16 == 0, "items behind the members stay aligned");
+    Item* items = (Item*)(d + mb);
+    float* cost = (float*)(items + n_items);
+    int16_t* grids = (int16_t*)(cost + n_items);
+    GB_CUDA_TRY(cudaMemcpyAsync(d, mi.data(), mb, cudaMemcpyHostToDevice, s));
+    k_merge_items<<<n, 256, 0, s>>>((const MemberItems*)d, items, cost, grids);
+    GB_CUDA_TRY(cudaGetLastError());
+    if ((rc = bundle_items(items, cost, grids, B->n_items, counts, B->cls, n, B->d_items,
+                           B->d_bundles, s)))
+      return rc;
+  }
   GB_CUDA_TRY(cudaStreamSynchronize(s));
   // the members' own piece tables are merged now: release them
   for (gb_plan* p : B->members) {
     cudaFree(p->d_recs);
     p->d_recs = nullptr;
+    p->release_raw();
     p->n_bundles = 0;  // a member can no longer run on its own FP32 tables
   }
   return GB_OK;

@@ -6,17 +6,21 @@
 // gridder's host std::sort (MS6/kernel/nvidia/gridder/binsort.cpp:6-35) with
 // a counting sort on the GPU:
 //   1. k_plan_count: per visibility, plane + index math (FP64), then a
-//      histogram of pieces per (tile, period rank);
-//   2. host: exclusive scan of the histogram, work items (record ranges of
-//      one tile and one thread-group class, cut by a cost model), bundles of
-//      items for the persistent kernels, longest first;
-//   3. k_plan_fill: recompute the index, scatter 16-byte records into their
-//      bins.
+//      histogram of pieces per (tile, period rank) and of visibilities per tile;
+//   2. an exclusive scan of both;
+//   3. k_plan_items, twice (count, write): work items, the record ranges of one
+//      tile and one thread-group class, cut by a cost model;
+//   4. k_plan_fill: 16-byte records scattered into their bins;
+//   5. bundle_items: items longest first, bundles of them for the persistent
+//      kernels, longest first.
+// The host reads back once, between counting and writing items, to size the
+// arrays.  1.17 M visibilities on a 4096^2 grid take 0.84 ms, of which the kernels
+// 0.28 ms (k_plan_count 110 us, its FP64 index math); with the scan, the items and
+// the bundles on the host 2.55 ms.  4.18 M: 1.04 ms (2.88), 4.18 M on 8192^2 1.25 ms
+// (6.39).
 #include <algorithm>
-#include <thread>
 #include <cstdlib>
 #include <cstring>
-#include <numeric>
 #include <vector>
 
 #include "gb_common.cuh"
@@ -25,111 +29,320 @@
 
 namespace gb {
 
-__global__ void k_plan_count(PlanDev P, const PlaneInfo* __restrict__ pl,
-                             const int32_t* __restrict__ plane_in, int32_t* __restrict__ plane_out,
-                             int32_t n_planes, double w_lo, double w_hi, int32_t T, int32_t ntx,
-                             int32_t nper, int32_t* __restrict__ hist,
-                             int32_t* __restrict__ vis_hist,
-                             unsigned long long* __restrict__ counters) {
-  __shared__ unsigned long long s_kept, s_taps, s_recs, s_paired;
-  if (threadIdx.x == 0) s_kept = s_taps = s_recs = s_paired = 0ull;
-  __syncthreads();
-  unsigned long long kept = 0, taps = 0, recs = 0, paired = 0;
+// What the plan's later kernels need of a visibility: its corner pixel and
+// phase (x < 0: not kept), so that the FP64 index math runs once.
+struct VisCell {
+  int32_t x, yp;  // yp = y | phase << 24 (a grid has at most 2^22 rows)
+};
+
+constexpr int kMaxRanks = 64;  // distinct periods
+
+// Counters of k_plan_count (the first four), k_rank_sums and k_plan_items, and
+// the classes' first items.
+struct PlanCounts {
+  unsigned long long kept, taps, recs, paired, tiles;
+  unsigned long long rank[kMaxRanks];  // pieces per period rank
+  int32_t class_first[kMaxClasses + 1];
+};
+
+// +1 at hist[key] for every active lane: one atomic per distinct key.  Returns
+// the lane's place among the key's lanes, in lane order, after what was there.
+__device__ __forceinline__ int32_t warp_count(int32_t* __restrict__ hist, int64_t key) {
+  const unsigned act = __activemask(), peers = __match_any_sync(act, key);
+  const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+  int32_t first = 0;
+  if (lane == leader) first = atomicAdd(&hist[key], __popc(peers));
+  first = __shfl_sync(act, first, leader);
+  return first + __popc(peers & ((1u << lane) - 1u));
+}
+
+__global__ void __launch_bounds__(256)
+    k_plan_count(PlanDev P, const PlaneInfo* __restrict__ pl, const int32_t* __restrict__ plane_in,
+                 int32_t* __restrict__ plane_out, VisCell* __restrict__ cells, int32_t n_planes,
+                 double w_lo, double w_hi, int32_t T, int32_t ntx, int32_t nper,
+                 int32_t* __restrict__ hist, int32_t* __restrict__ vis_hist,
+                 PlanCounts* __restrict__ cnt) {
+  unsigned long long sum[4] = {0, 0, 0, 0};  // kept, taps, recs, paired
+  const int64_t ntiles = (int64_t)ntx * ((P.ext_y + T - 1) / T);
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < P.n_vis;
        t += (int64_t)gridDim.x * blockDim.x) {
     const double* r = P.uvw + t * P.uvw_stride;
     int32_t p = plane_in ? plane_in[t] : w_plane(r[2], w_lo, w_hi, n_planes);
     if (p >= n_planes) p = -1;
     plane_out[t] = p;
-    const int64_t ntiles = (int64_t)ntx * ((P.ext_y + T - 1) / T);
-    if (p < 0) {
-      atomicAdd(&vis_hist[ntiles], 1);  // skipped visibilities go last
-      continue;
+    VisIndex ix;
+    ix.keep = false;
+    PlaneInfo q;
+    if (p >= 0) {
+      q = pl[p];
+      ix = vis_index(r[0], r[1], P.scale, P.grid_size, q.S, P.margin, 0, 0, P.ext_x, P.ext_y);
     }
-    const PlaneInfo q = pl[p];
-    const VisIndex ix =
-        vis_index(r[0], r[1], P.scale, P.grid_size, q.S, P.margin, 0, 0, P.ext_x, P.ext_y);
-    if (!ix.keep) {
-      atomicAdd(&vis_hist[ntiles], 1);
-      continue;
-    }
-    atomicAdd(&vis_hist[(int64_t)(ix.y0 / T) * ntx + ix.x0 / T], 1);
-    kept++;
-    taps += (unsigned long long)q.S * q.S;
-    for (int ky = 0; ky < q.k; ky++) {
-      const int Y0 = ix.y0 + ky * q.P;
-      if (ky * q.P >= q.S) break;
-      for (int kx = 0; kx < q.k; kx++) {
-        if (kx * q.P >= q.S) break;
-        const int X0 = ix.x0 + kx * q.P;
-        const int64_t tile = (int64_t)(Y0 / T) * ntx + (X0 / T);
-        atomicAdd(&hist[tile * nper + q.rank], 1);
-        recs++;
+    cells[t] = ix.keep ? VisCell{ix.x0, ix.y0 | ix.phase << 24} : VisCell{-1, 0};
+    // skipped visibilities go last
+    warp_count(vis_hist, ix.keep ? (int64_t)(ix.y0 / T) * ntx + ix.x0 / T : ntiles);
+    if (!ix.keep) continue;
+    sum[0]++;
+    sum[1] += (unsigned long long)q.S * q.S;
+    for (int oy = 0; oy < q.S; oy += q.P) {
+      const int64_t row = (int64_t)((ix.y0 + oy) / T) * ntx;
+      for (int ox = 0; ox < q.S; ox += q.P) {
+        warp_count(hist, (row + (ix.x0 + ox) / T) * nper + q.rank);
+        sum[2]++;
         // degridding pairs the taps of a piece whose rows, GCF rows and GCF
         // offset are all even (the same rule the kernels apply per record)
-        const int wx = min(q.P, q.S - kx * q.P), wy = min(q.P, q.S - ky * q.P);
-        if (((wx | q.S | (int)((q.gcf_off + kx * q.P) & 1)) & 1) == 0)
-          paired += (unsigned long long)wx * wy;
+        const int wx = min(q.P, q.S - ox), wy = min(q.P, q.S - oy);
+        if (((wx | q.S | (int)((q.gcf_off + ox) & 1)) & 1) == 0)
+          sum[3] += (unsigned long long)wx * wy;
       }
     }
   }
-  atomicAdd(&s_kept, kept);
-  atomicAdd(&s_taps, taps);
-  atomicAdd(&s_recs, recs);
-  atomicAdd(&s_paired, paired);
+  __shared__ unsigned long long s_sum[8][4];  // per warp
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5][k] = sum[k];
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    atomicAdd(&counters[0], s_kept);
-    atomicAdd(&counters[1], s_taps);
-    atomicAdd(&counters[2], s_recs);
-    atomicAdd(&counters[3], s_paired);
+  if (threadIdx.x < 4) {
+    unsigned long long all = 0;
+    for (int w = 0; w < 8; w++) all += s_sum[w][threadIdx.x];
+    if (all) atomicAdd(&cnt->kept + threadIdx.x, all);
   }
 }
 
-__global__ void k_plan_fill(PlanDev P, const PlaneInfo* __restrict__ pl, int32_t T, int32_t ntx,
-                            int32_t nper, const int32_t* __restrict__ offs,
-                            int32_t* __restrict__ cursor, Rec* __restrict__ recs,
-                            const int32_t* __restrict__ vis_offs,
+// Pieces per period rank (keys run rank-fastest within a tile).
+__global__ void __launch_bounds__(256) k_rank_sums(const int32_t* __restrict__ hist, int64_t nkeys,
+                                                   int nper, PlanCounts* __restrict__ cnt) {
+  __shared__ unsigned long long s_rank[kMaxRanks];
+  for (int r = threadIdx.x; r < nper; r += blockDim.x) s_rank[r] = 0;
+  __syncthreads();
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nkeys;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t v = hist[i];
+    if (v) atomicAdd(&s_rank[i % nper], (unsigned long long)v);
+  }
+  __syncthreads();
+  for (int r = threadIdx.x; r < nper; r += blockDim.x)
+    if (s_rank[r]) atomicAdd(&cnt->rank[r], s_rank[r]);
+}
+
+// ---------------------------------------------------------------- exclusive scan
+// out[i] = in[0] + .. + in[i - 1] for i = 0 .. n, modulo 2^32: sums per block of
+// kScanKeys keys, their scan by one block, the keys' scan with those.
+constexpr int kScanThreads = 512, kScanPer = 8, kScanKeys = kScanThreads * kScanPer;
+
+// Exclusive scan over the block of each thread's value; *total the sum.
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* total) {
+  __shared__ uint32_t warp_sum[kScanThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t a = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += a;
+  }
+  __syncthreads();  // warp_sum of an earlier call is read
+  if (lane == 31) warp_sum[warp] = inc;
+  __syncthreads();
+  uint32_t before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < kScanThreads / 32; w++) {
+    if (w < warp) before += warp_sum[w];
+    all += warp_sum[w];
+  }
+  *total = all;
+  return before + inc - v;
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+    k_scan_sums(const int32_t* __restrict__ in, int64_t n, uint32_t* __restrict__ sums) {
+  const int64_t i0 = (int64_t)blockIdx.x * kScanKeys;
+  uint32_t v = 0;
+#pragma unroll
+  for (int k = 0; k < kScanPer; k++) {
+    const int64_t i = i0 + k * kScanThreads + threadIdx.x;
+    if (i < n) v += (uint32_t)in[i];
+  }
+  uint32_t total;
+  block_scan(v, &total);
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_scan_top(uint32_t* __restrict__ sums, int nb) {
+  uint32_t carry = 0;
+  for (int b = 0; b < nb; b += kScanThreads) {
+    const int i = b + threadIdx.x;
+    const uint32_t v = i < nb ? sums[i] : 0u;
+    uint32_t total;
+    const uint32_t e = block_scan(v, &total);
+    if (i < nb) sums[i] = carry + e;
+    carry += total;
+  }
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+    k_scan_keys32(const int32_t* __restrict__ in, int64_t n, const uint32_t* __restrict__ sums,
+                  int32_t* __restrict__ out) {
+  const int64_t i0 = (int64_t)blockIdx.x * kScanKeys + (int64_t)threadIdx.x * kScanPer;
+  uint32_t v[kScanPer], sum = 0;
+#pragma unroll
+  for (int k = 0; k < kScanPer; k++) {
+    v[k] = i0 + k < n ? (uint32_t)in[i0 + k] : 0u;
+    sum += v[k];
+  }
+  uint32_t total, e = block_scan(sum, &total) + sums[blockIdx.x];
+#pragma unroll
+  for (int k = 0; k < kScanPer; k++) {
+    if (i0 + k <= n) out[i0 + k] = (int32_t)e;
+    e += v[k];
+  }
+}
+
+static int64_t scan_blocks(int64_t n) { return n / kScanKeys + 1; }  // out has n + 1 entries
+
+// sums: scan_blocks(n) words of scratch.
+static int scan_keys(const int32_t* in, int64_t n, int32_t* out, uint32_t* sums, cudaStream_t s) {
+  const int nb = (int)scan_blocks(n);
+  k_scan_sums<<<nb, kScanThreads, 0, s>>>(in, n, sums);
+  k_scan_top<<<1, kScanThreads, 0, s>>>(sums, nb);
+  k_scan_keys32<<<nb, kScanThreads, 0, s>>>(in, n, sums, out);
+  GB_CUDA_TRY(cudaGetLastError());
+  return GB_OK;
+}
+
+// ---------------------------------------------------------------- items
+// How the items are cut: the classes' period ranks (consecutive: group width
+// grows with the period), the cost of a record and of an item, and per rank the
+// split-row stride residue of degridding.
+struct ItemRule {
+  int nper, nclass;
+  int lo[kMaxClasses], hi[kMaxClasses];
+  float fixed[kMaxClasses];
+  float rec[kMaxRanks];       // cost of a record
+  double per_cta[kMaxRanks];  // the same over the items a CTA runs side by side
+  int16_t period[kMaxRanks];
+  int8_t residue[kMaxRanks];
+  double pieces;  // items wanted per unit of total cost: bundles per CTA x CTAs
+};
+
+// The items of each (class, tile): counted (per class, tile-fastest), or with
+// `items` written from first[] on.  An item is closed when its cost reaches the
+// larger of four times its fixed cost and an even share of all the work.
+__global__ void __launch_bounds__(128)
+    k_plan_items(const __grid_constant__ ItemRule R, int64_t ntiles, int32_t ntx,
+                 const int32_t* __restrict__ offs, PlanCounts* __restrict__ cnt,
+                 int32_t* __restrict__ count, const int32_t* __restrict__ first,
+                 Item* __restrict__ items, float* __restrict__ costs) {
+  __shared__ float s_tau;
+  if (threadIdx.x == 0) {
+    double total = 0;
+    for (int r = 0; r < R.nper; r++) total += (double)cnt->rank[r] * R.per_cta[r];
+    s_tau = (float)(total / R.pieces);
+  }
+  __syncthreads();
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int c = (int)(e / ntiles);
+  const int64_t tile = e - c * ntiles;
+  bool used = false;
+  if (c < R.nclass) {
+    const int64_t k0 = tile * R.nper;
+    const int32_t b0 = offs[k0 + R.lo[c]], b1 = offs[k0 + R.hi[c]];
+    used = c == 0 && offs[k0 + R.nper] != offs[k0];
+    int n = 0;
+    if (b1 != b0) {
+      int64_t at = items ? first[e] : 0;
+      const float fixed = R.fixed[c], cmax = fmaxf(4.f * fixed, s_tau);
+      float cost = fixed;
+      int32_t start = b0, in_item = 0;
+      int64_t top_taps = 0;
+      int top = -1, pmax = 0;
+      auto close = [&]() {
+        if (items) {
+          Item it;
+          it.start = start;
+          it.count = in_item;
+          it.tile_x = (int16_t)(tile % ntx);
+          it.tile_y = (int16_t)(tile / ntx);
+          it.pmax = (int16_t)pmax;
+          it.cls = item_cls_with_residue((int16_t)c, R.residue[top]);
+          items[at] = it;
+          costs[at] = cost;
+          at++;
+        }
+        n++;
+        start += in_item;
+        in_item = 0;
+        cost = fixed;
+        top_taps = 0;
+        pmax = 0;
+      };
+      for (int r = R.lo[c]; r < R.hi[c]; r++) {
+        int32_t pos = offs[k0 + r];
+        const int32_t end = offs[k0 + r + 1];
+        const float rc = R.rec[r], per = 1.f / rc;
+        while (pos < end) {
+          const float room = fminf((cmax - cost) * per, 2e9f);
+          const int32_t take = min(max((int32_t)room, 1), end - pos);
+          const int64_t t = (int64_t)take * R.period[r] * R.period[r];
+          if (t > top_taps) {  // the stage stride goes by the largest run
+            top_taps = t;
+            top = r;
+          }
+          pmax = R.period[r];
+          in_item += take;
+          cost += (float)take * rc;
+          pos += take;
+          if (cost >= cmax) close();
+        }
+      }
+      if (in_item) close();
+    }
+    if (!items) count[e] = n;
+  }
+  if (!items) {
+    const int used_here = __syncthreads_count(used);
+    if (threadIdx.x == 0 && used_here) atomicAdd(&cnt->tiles, (unsigned long long)used_here);
+  }
+}
+
+// The classes' first items, from the scan of their counts.
+__global__ void k_plan_classes(const int32_t* __restrict__ first, int64_t ntiles, int nclass,
+                               PlanCounts* __restrict__ cnt) {
+  if (threadIdx.x <= nclass) cnt->class_first[threadIdx.x] = first[threadIdx.x * ntiles];
+}
+
+// offs, vis_offs: the scan of both histograms one after the other; the cursors
+// are the same arrays, zeroed again.
+__global__ void k_plan_fill(PlanDev P, const PlaneInfo* __restrict__ pl,
+                            const VisCell* __restrict__ cells, int32_t T, int32_t ntx, int32_t nper,
+                            const int32_t* __restrict__ offs, int32_t* __restrict__ cursor,
+                            Rec* __restrict__ recs, const int32_t* __restrict__ vis_offs,
                             int32_t* __restrict__ vis_cursor, int32_t* __restrict__ order) {
   const int64_t ntiles = (int64_t)ntx * ((P.ext_y + T - 1) / T);
+  const uint32_t vis0 = (uint32_t)vis_offs[0];
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < P.n_vis;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t p = P.plane[t];
-    if (p < 0) {
-      order[vis_offs[ntiles] + atomicAdd(&vis_cursor[ntiles], 1)] = (int32_t)t;
-      continue;
-    }
-    const PlaneInfo q = pl[p];
-    const double* r = P.uvw + t * P.uvw_stride;
-    const VisIndex ix =
-        vis_index(r[0], r[1], P.scale, P.grid_size, q.S, P.margin, 0, 0, P.ext_x, P.ext_y);
-    const int64_t vt = ix.keep ? (int64_t)(ix.y0 / T) * ntx + ix.x0 / T : ntiles;
-    order[vis_offs[vt] + atomicAdd(&vis_cursor[vt], 1)] = (int32_t)t;
-    if (!ix.keep) continue;
-    const int64_t gbase = q.gcf_off + (int64_t)ix.phase * q.S * q.S;
-    for (int ky = 0; ky < q.k; ky++) {
-      const int oy = ky * q.P;
-      if (oy >= q.S) break;
-      const int Y0 = ix.y0 + oy;
+    const VisCell cell = cells[t];
+    const bool keep = cell.x >= 0;
+    const int x0 = cell.x, y0 = cell.yp & 0xFFFFFF, phase = cell.yp >> 24;
+    const int64_t vt = keep ? (int64_t)(y0 / T) * ntx + x0 / T : ntiles;
+    order[(uint32_t)vis_offs[vt] - vis0 + (uint32_t)warp_count(vis_cursor, vt)] = (int32_t)t;
+    if (!keep) continue;
+    const PlaneInfo q = pl[P.plane[t]];
+    const int64_t gbase = q.gcf_off + (int64_t)phase * q.S * q.S;
+    for (int oy = 0; oy < q.S; oy += q.P) {
+      const int Y0 = y0 + oy, ty = Y0 / T;
       const int wy = min(q.P, q.S - oy);
-      for (int kx = 0; kx < q.k; kx++) {
-        const int ox = kx * q.P;
-        if (ox >= q.S) break;
-        const int X0 = ix.x0 + ox;
+      for (int ox = 0; ox < q.S; ox += q.P) {
+        const int X0 = x0 + ox, tx = X0 / T;
         const int wx = min(q.P, q.S - ox);
-        const int tx = X0 / T, ty = Y0 / T;
+        // lanes with the same bin take consecutive places in lane order:
+        // neighbouring samples of a baseline, which a warp holds side by side,
+        // stay neighbours in the bin, where the gridder sums the taps that
+        // consecutive pieces put on one pixel
         const int64_t key = ((int64_t)ty * ntx + tx) * nper + q.rank;
-        // lanes with the same bin take consecutive places in lane order (one
-        // atomic per bin and warp): neighbouring samples of a baseline, which
-        // a warp holds side by side, stay neighbours in the bin, where the
-        // gridder sums the taps that consecutive pieces put on one pixel
-        const unsigned act = __activemask();
-        const unsigned peers = __match_any_sync(act, key);
-        const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
-        int32_t first = 0;
-        if (lane == leader) first = atomicAdd(&cursor[key], __popc(peers));
-        first = __shfl_sync(act, first, leader);
-        const int32_t pos = offs[key] + first + __popc(peers & ((1u << lane) - 1u));
+        const int32_t pos = offs[key] + warp_count(cursor, key);
         Rec rc;
         rc.vis = (int32_t)t;
         rc.gcf = (uint32_t)(gbase + (int64_t)oy * q.S + ox);
@@ -145,6 +358,144 @@ __global__ void k_plan_fill(PlanDev P, const PlaneInfo* __restrict__ pl, int32_t
       }
     }
   }
+}
+
+// ---------------------------------------------------------------- bundles
+// Items sorted by cost within their (class, grid) bucket, quantised to kLevels
+// levels of the largest cost (the longest-first heuristic needs no finer
+// order), groups of G of them as bundles, bundles sorted likewise.
+constexpr int kLevels = 1024;
+
+struct Bucket {
+  int32_t first, count, first_bundle, G;
+};
+
+__global__ void k_cost_max(const float* __restrict__ cost, int n, int* __restrict__ top) {
+  float m = 0.f;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    m = fmaxf(m, cost[i]);
+  const int w = __reduce_max_sync(0xffffffffu, __float_as_int(m));
+  if ((threadIdx.x & 31) == 0) atomicMax(top, w);
+}
+
+__device__ __forceinline__ int cost_level(float cost, const int* top) {
+  const float m = __int_as_float(*top);
+  const int l = m > 0.f ? (int)(cost / m * (kLevels - 1)) : 0;
+  return kLevels - 1 - min(max(l, 0), kLevels - 1);  // largest first
+}
+
+__device__ __forceinline__ int64_t item_key(const Item& it, int grid, int ngrid, int level) {
+  return ((int64_t)item_class(it.cls) * ngrid + grid) * kLevels + level;
+}
+
+// grids: the items' grid slots, or NULL (slot 0).
+__global__ void k_item_levels(const Item* __restrict__ items, const float* __restrict__ cost,
+                              const int16_t* __restrict__ grids, int n, int ngrid,
+                              const int* __restrict__ top, int32_t* __restrict__ hist) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n)
+    warp_count(hist, item_key(items[i], grids ? grids[i] : 0, ngrid, cost_level(cost[i], top)));
+}
+
+__global__ void k_item_place(const Item* __restrict__ items, const float* __restrict__ cost,
+                             const int16_t* __restrict__ grids, int n, int ngrid,
+                             const int* __restrict__ top, const int32_t* __restrict__ offs,
+                             int32_t* __restrict__ cursor, Item* __restrict__ out,
+                             int32_t* __restrict__ levels) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int level = cost_level(cost[i], top);
+  const int64_t key = item_key(items[i], grids ? grids[i] : 0, ngrid, level);
+  const int pos = offs[key] + warp_count(cursor, key);
+  out[pos] = items[i];
+  levels[pos] = level;
+}
+
+__device__ __forceinline__ int find_bucket(const Bucket* __restrict__ b, int n, int bundle) {
+  int lo = 0, hi = n - 1;  // the last bucket whose first bundle is not after it
+  while (lo < hi) {
+    const int m = (lo + hi + 1) / 2;
+    if (b[m].first_bundle <= bundle)
+      lo = m;
+    else
+      hi = m - 1;
+  }
+  return lo;
+}
+
+// Counts the bundles' levels, or with `out` writes them in level order.
+__global__ void k_bundles(const Bucket* __restrict__ buckets, int nbuckets, int ngrid, int n,
+                          const int32_t* __restrict__ levels, int32_t* __restrict__ hist,
+                          const int32_t* __restrict__ offs, Bundle* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int k = find_bucket(buckets, nbuckets, i);
+  const Bucket b = buckets[k];
+  const int at = (i - b.first_bundle) * b.G, level = levels[b.first + at];
+  const int place = warp_count(hist, level);
+  if (!out) return;
+  Bundle q;
+  q.first_item = b.first + at;
+  q.n_items = (int16_t)min(b.G, b.count - at);
+  q.cls = (int16_t)(k / ngrid);
+  q.grid = k % ngrid;
+  q.pad = 0;
+  out[offs[level] + place] = q;
+}
+
+int count_bundles(const std::vector<int>& counts, const ClassInfo* cls, int ngrid) {
+  int64_t n = 0;
+  for (size_t k = 0; k < counts.size(); k++) {
+    const int G = cls[k / ngrid].G;
+    n += (counts[k] + G - 1) / G;
+  }
+  return (int)n;
+}
+
+int bundle_items(const Item* items, const float* cost, const int16_t* grids, int n,
+                 const std::vector<int>& counts, const ClassInfo* cls, int ngrid, Item* out,
+                 Bundle* bundles, cudaStream_t s) {
+  if (n == 0) return GB_OK;
+  const int nb = (int)counts.size();
+  std::vector<Bucket> hb(nb);
+  int first = 0, fb = 0;
+  for (int k = 0; k < nb; k++) {
+    hb[k] = Bucket{first, counts[k], fb, cls[k / ngrid].G};
+    first += counts[k];
+    fb += (counts[k] + hb[k].G - 1) / hb[k].G;
+  }
+  const int64_t keys = (int64_t)nb * kLevels;
+  // scratch: top | item histogram | bundle histogram (zeroed), their scans, the
+  // items' levels, scan sums, buckets
+  const int64_t zero = 1 + keys + kLevels;
+  const int64_t words = 2 * zero + 3 + n + scan_blocks(keys) + 4 * (int64_t)nb;
+  int32_t* d = nullptr;
+  int rc = dev_alloc((void**)&d, sizeof(int32_t) * words, "plan bundles");
+  if (rc) return rc;
+  int *top = d, *hist = top + 1, *bhist = hist + keys;
+  int *offs = d + zero, *boffs = offs + keys + 1, *levels = boffs + kLevels + 1;
+  uint32_t* sums = (uint32_t*)(levels + n);
+  Bucket* db = (Bucket*)(sums + scan_blocks(keys));
+  const int ib = (n + 255) / 256, bb = (fb + 255) / 256;
+  auto run = [&]() -> int {
+    GB_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(int32_t) * zero, s));
+    GB_CUDA_TRY(cudaMemcpyAsync(db, hb.data(), sizeof(Bucket) * nb, cudaMemcpyHostToDevice, s));
+    k_cost_max<<<std::min(ib, sm_count()), 256, 0, s>>>(cost, n, top);
+    k_item_levels<<<ib, 256, 0, s>>>(items, cost, grids, n, ngrid, top, hist);
+    if ((rc = scan_keys(hist, keys, offs, sums, s))) return rc;
+    GB_CUDA_TRY(cudaMemsetAsync(hist, 0, sizeof(int32_t) * keys, s));
+    k_item_place<<<ib, 256, 0, s>>>(items, cost, grids, n, ngrid, top, offs, hist, out, levels);
+    k_bundles<<<bb, 256, 0, s>>>(db, nb, ngrid, fb, levels, bhist, nullptr, nullptr);
+    if ((rc = scan_keys(bhist, kLevels, boffs, sums, s))) return rc;
+    GB_CUDA_TRY(cudaMemsetAsync(bhist, 0, sizeof(int32_t) * kLevels, s));
+    k_bundles<<<bb, 256, 0, s>>>(db, nb, ngrid, fb, levels, bhist, boffs, bundles);
+    GB_CUDA_TRY(cudaGetLastError());
+    GB_CUDA_TRY(cudaStreamSynchronize(s));
+    return GB_OK;
+  };
+  rc = run();
+  cudaFree(d);
+  return rc;
 }
 
 __global__ void k_plan_export(PlanDev P, const int32_t* __restrict__ supports,
@@ -185,17 +536,22 @@ static int blocks_for(int64_t n, int threads) {
   return (int)(b < 1 ? 1 : b);
 }
 
+}  // namespace gb
+
+void gb_plan::release_raw() {
+  cudaFree(d_raw_items);
+  d_raw_items = nullptr;
+  d_raw_cost = nullptr;
+}
+
+namespace gb {
+
 static void free_plan(gb_plan* p) {
   if (!p) return;
-  cudaFree(p->d_plane);
-  cudaFree(p->d_order);
-  cudaFree(p->d_supports);
-  cudaFree(p->d_offsets);
-  cudaFree(p->d_planes);
+  cudaFree(p->d_tables);
   cudaFree(p->d_recs);
   cudaFree(p->d_items);
-  cudaFree(p->d_bundles);
-  cudaFree(p->d_queue);
+  p->release_raw();
   p->df.release();
   delete p;
 }
@@ -206,85 +562,6 @@ static int dalloc(T** p, size_t n) {
   const int rc = dev_alloc(&q, sizeof(T) * (n ? n : 1), "plan");
   *p = (T*)q;
   return rc;
-}
-
-// idx[0..n) reordered by cost, largest first, in one counting pass over the
-// costs quantised to 4096 levels of the largest (ties keep their order): the
-// longest-first heuristic needs no finer order, and a comparison sort of tens
-// of thousands of items costs milliseconds of host time per plan.
-static void order_by_cost(const std::vector<double>& cost, int32_t* idx, size_t n) {
-  if (n < 2) return;
-  constexpr int K = 4096;
-  double top = 0;
-  for (size_t i = 0; i < n; i++) top = std::max(top, cost[idx[i]]);
-  const double q = top > 0 ? (K - 1) / top : 0.0;
-  std::vector<int32_t> cnt(K + 1, 0), tmp(idx, idx + n);
-  auto level = [&](int32_t i) {
-    const int l = (int)(cost[i] * q);
-    return K - 1 - std::min(std::max(l, 0), K - 1);  // largest first
-  };
-  for (size_t i = 0; i < n; i++) cnt[level(tmp[i]) + 1]++;
-  for (int k = 1; k <= K; k++) cnt[k] += cnt[k - 1];
-  for (size_t i = 0; i < n; i++) idx[cnt[level(tmp[i])]++] = tmp[i];
-}
-
-void make_bundles(const std::vector<HostItem>& items, const ClassInfo* cls, int n_classes,
-                  std::vector<Item>& it_out, std::vector<Bundle>& b_out) {
-  // items by (class, grid slot), each bucket in the items' own order: one
-  // counting pass (a batch has up to kMaxGrids slots)
-  int max_grid = 0;
-  for (const auto& h : items) max_grid = std::max(max_grid, h.grid);
-  const size_t ng = (size_t)max_grid + 1, nb = (size_t)n_classes * ng;
-  std::vector<size_t> first(nb + 1, 0);
-  for (const auto& h : items) first[(size_t)item_class(h.it.cls) * ng + h.grid + 1]++;
-  for (size_t k = 1; k <= nb; k++) first[k] += first[k - 1];
-  std::vector<int32_t> order(items.size());
-  {
-    std::vector<size_t> next(first.begin(), first.end() - 1);
-    for (size_t i = 0; i < items.size(); i++)
-      order[next[(size_t)item_class(items[i].it.cls) * ng + items[i].grid]++] = (int32_t)i;
-  }
-  // within a bucket, longest first; groups of G items form a bundle
-  struct HB {
-    Bundle b;
-    double cost;
-  };
-  std::vector<HB> bundles;
-  bundles.reserve(items.size());
-  it_out.clear();
-  it_out.reserve(items.size());
-  std::vector<double> cost(items.size());
-  for (size_t i = 0; i < items.size(); i++) cost[i] = items[i].cost;
-  for (int c = 0; c < n_classes; c++) {
-    const int G = cls[c].G;
-    for (size_t g = 0; g < ng; g++) {
-      const size_t k = (size_t)c * ng + g;
-      if (first[k] == first[k + 1]) continue;
-      order_by_cost(cost, order.data() + first[k], first[k + 1] - first[k]);
-      for (size_t i = first[k]; i < first[k + 1]; i += G) {
-        HB hb;
-        hb.b.first_item = (int32_t)it_out.size();
-        hb.b.n_items = (int16_t)std::min<size_t>(G, first[k + 1] - i);
-        hb.b.cls = (int16_t)c;
-        hb.b.grid = (int32_t)g;
-        hb.b.pad = 0;
-        hb.cost = items[order[i]].cost;
-        for (int m = 0; m < hb.b.n_items; m++) it_out.push_back(items[order[i + m]].it);
-        bundles.push_back(hb);
-      }
-    }
-  }
-  // all bundles, longest first
-  std::vector<int32_t> bo(bundles.size());
-  std::vector<double> bcost(bundles.size());
-  for (size_t i = 0; i < bo.size(); i++) {
-    bo[i] = (int32_t)i;
-    bcost[i] = bundles[i].cost;
-  }
-  order_by_cost(bcost, bo.data(), bo.size());
-  b_out.clear();
-  b_out.reserve(bundles.size());
-  for (int32_t i : bo) b_out.push_back(bundles[i].b);
 }
 
 // Modelled shared-memory wavefronts per pair that degridding's split-row stage
@@ -375,11 +652,24 @@ static int build_plan(gb_plan* P, const gb_geometry* geo, int64_t n_vis, const d
   for (int st = 0; st < 3; st++) P->ctas_per_sm_degrid[st] = tiled_ctas_per_sm(P, false, st);
 
   // ---- device tables
-  if ((rc = dalloc(&P->d_plane, n_vis)) || (rc = dalloc(&P->d_order, n_vis)) ||
-      (rc = dalloc(&P->d_supports, np)) ||
-      (rc = dalloc(&P->d_offsets, np)) || (rc = dalloc(&P->d_planes, np)) ||
-      (rc = dalloc(&P->d_queue, 3)))
-    return rc;
+  {
+    size_t bytes = 0;
+    auto place = [&](size_t n) {
+      const size_t at = bytes;
+      bytes += (n + 255) & ~(size_t)255;
+      return at;
+    };
+    const size_t plane = place(sizeof(int32_t) * n_vis), order = place(sizeof(int32_t) * n_vis);
+    const size_t sup = place(sizeof(int32_t) * np), offs = place(sizeof(int64_t) * np);
+    const size_t planes = place(sizeof(PlaneInfo) * np), queue = place(sizeof(int32_t) * 3);
+    if ((rc = dalloc(&P->d_tables, bytes))) return rc;
+    P->d_plane = (int32_t*)(P->d_tables + plane);
+    P->d_order = (int32_t*)(P->d_tables + order);
+    P->d_supports = (int32_t*)(P->d_tables + sup);
+    P->d_offsets = (int64_t*)(P->d_tables + offs);
+    P->d_planes = (PlaneInfo*)(P->d_tables + planes);
+    P->d_queue = (int32_t*)(P->d_tables + queue);
+  }
   // [0], [1]: work-queue heads of the grid and degrid kernels; [2]: device
   // error word (a TMA stage completion not seen in time)
   GB_CUDA_TRY(cudaMemsetAsync(P->d_queue, 0, 3 * sizeof(int32_t), s));
@@ -413,235 +703,130 @@ static int build_plan(gb_plan* P, const gb_geometry* geo, int64_t n_vis, const d
     return GB_ERR_CAPACITY;
   }
   // per-visibility order: one bucket per tile (the footprint corner's) and a
-  // last one for the visibilities no kernel grids
-  const int64_t nvkeys = (int64_t)P->ntx * P->nty + 1;
-  int32_t *d_hist = nullptr, *d_offs = nullptr, *d_vhist = nullptr, *d_voffs = nullptr;
-  unsigned long long* d_cnt = nullptr;
-  if ((rc = dalloc(&d_hist, nkeys)) || (rc = dalloc(&d_offs, nkeys + 1)) ||
-      (rc = dalloc(&d_vhist, nvkeys)) || (rc = dalloc(&d_voffs, nvkeys)) ||
-      (rc = dalloc(&d_cnt, 4))) {
-    cudaFree(d_hist);
-    cudaFree(d_offs);
-    cudaFree(d_vhist);
-    cudaFree(d_voffs);
-    cudaFree(d_cnt);
-    return rc;
-  }
+  // last one for the visibilities no kernel grids; both histograms lie one
+  // after the other and are scanned together
+  const int64_t ntiles = (int64_t)P->ntx * P->nty, nvkeys = ntiles + 1, all = nkeys + nvkeys;
+  const int64_t nci = ntiles * P->n_classes;
+  const int64_t nsums = std::max(scan_blocks(all), scan_blocks(nci));
+  // scratch: counters and histograms (zeroed), their scan, the items' counts and
+  // scan, scan sums, the visibilities' cells
+  const size_t cnt_bytes = (sizeof(PlanCounts) + 255) & ~(size_t)255;
+  const size_t words = (size_t)(all + (all + 1) + nci + (nci + 1) + nsums + 1) & ~(size_t)1;
+  unsigned char* d = nullptr;
+  if ((rc = dalloc(&d, cnt_bytes + sizeof(int32_t) * words + sizeof(VisCell) * n_vis))) return rc;
   struct Tmp {
-    void* p[5];
-    ~Tmp() {
-      for (void* q : p) cudaFree(q);
-    }
-  } tmp{{d_hist, d_offs, d_vhist, d_voffs, d_cnt}};
-  GB_CUDA_TRY(cudaMemsetAsync(d_hist, 0, sizeof(int32_t) * nkeys, s));
-  GB_CUDA_TRY(cudaMemsetAsync(d_vhist, 0, sizeof(int32_t) * nvkeys, s));
-  GB_CUDA_TRY(cudaMemsetAsync(d_cnt, 0, sizeof(unsigned long long) * 4, s));
+    void* p;
+    ~Tmp() { cudaFree(p); }
+  } tmp{d};
+  PlanCounts* d_cnt = (PlanCounts*)d;
+  int32_t* d_hist = (int32_t*)(d + cnt_bytes);
+  int32_t* d_vhist = d_hist + nkeys;
+  int32_t* d_offs = d_hist + all;
+  int32_t* d_icount = d_offs + all + 1;
+  int32_t* d_ifirst = d_icount + nci;
+  uint32_t* d_sums = (uint32_t*)(d_ifirst + nci + 1);
+  VisCell* d_cells = (VisCell*)(d_hist + words);
+  GB_CUDA_TRY(cudaMemsetAsync(d, 0, cnt_bytes + sizeof(int32_t) * all, s));
   if (n_vis > 0) {
-    k_plan_count<<<blocks_for(n_vis, 256), 256, 0, s>>>(
-        D, P->d_planes, d_plane_in, P->d_plane, np, geo->w_low, geo->w_high, P->T, P->ntx, nper,
-        d_hist, d_vhist, d_cnt);
+    const int blocks = std::min(blocks_for(n_vis, 256), sm_count() * 8);
+    k_plan_count<<<blocks, 256, 0, s>>>(
+        D, P->d_planes, d_plane_in, P->d_plane, d_cells, np, geo->w_low, geo->w_high, P->T, P->ntx,
+        nper, d_hist, d_vhist, d_cnt);
+    k_rank_sums<<<blocks_for(nkeys, 4096), 256, 0, s>>>(d_hist, nkeys, nper, d_cnt);
     GB_CUDA_TRY(cudaGetLastError());
   }
-  std::vector<int32_t> hist(nkeys), vhist(nvkeys);
-  unsigned long long cnt[4];
-  GB_CUDA_TRY(cudaMemcpyAsync(hist.data(), d_hist, sizeof(int32_t) * nkeys, cudaMemcpyDeviceToHost,
-                              s));
-  GB_CUDA_TRY(cudaMemcpyAsync(vhist.data(), d_vhist, sizeof(int32_t) * nvkeys,
-                              cudaMemcpyDeviceToHost, s));
-  GB_CUDA_TRY(cudaMemcpyAsync(cnt, d_cnt, sizeof(cnt), cudaMemcpyDeviceToHost, s));
-  GB_CUDA_TRY(cudaStreamSynchronize(s));
-  P->kept = (int64_t)cnt[0];
-  P->taps = (int64_t)cnt[1];
-  P->n_recs = (int64_t)cnt[2];
-  P->taps_paired = (int64_t)cnt[3];
-  if (P->n_recs >= (int64_t)INT32_MAX) {
-    gb_set_error(GB_ERR_CAPACITY, "more than 2^31 footprint pieces");
-    return GB_ERR_CAPACITY;
-  }
-
-  // ---- scan + items
-  std::vector<int32_t> offs(nkeys + 1);
-  int64_t acc = 0;
-  for (int64_t k = 0; k < nkeys; k++) {
-    offs[k] = (int32_t)acc;
-    acc += hist[k];
-  }
-  offs[nkeys] = (int32_t)acc;
+  if ((rc = scan_keys(d_hist, all, d_offs, d_sums, s))) return rc;
 
   // cost model, in thread-group steps: a piece of period P costs ceil(P^2/L)
   // tap rounds plus one for its record; an item adds zeroing + flush of its
   // A x A accumulator.
-  std::vector<double> rec_cost(nper);
-  for (int r = 0; r < nper; r++) {
-    const int L = P->cls[rank_cls[r]].L;
-    rec_cost[r] = (double)((periods[r] * periods[r] + L - 1) / L + 1);
-  }
-  auto fixed_cost = [&](int c) {
+  ItemRule R{};
+  R.nper = nper;
+  R.nclass = P->n_classes;
+  for (int c = 0; c < P->n_classes; c++) {
     const ClassInfo& ci = P->cls[c];
-    return (double)(2 * ((ci.A * ci.A + ci.L - 1) / ci.L));
-  };
-  // the histogram's cost per CTA slot (keys run rank-fastest within a tile)
-  std::vector<double> rank_w(nper);
-  for (int r = 0; r < nper; r++) rank_w[r] = rec_cost[r] / P->cls[rank_cls[r]].G;
-  double total_cta = 0;
-  for (int64_t k0 = 0; k0 < nkeys; k0 += nper)
-    for (int r = 0; r < nper; r++) total_cta += hist[k0 + r] * rank_w[r];
-  const int ctas = std::max(1, sm_count() * std::max(1, P->ctas_per_sm_grid));
-  const double tau = total_cta / ((double)P->bpc * ctas);
-  // a class's periods are consecutive ranks (group width grows with the period)
-  std::vector<int> r_lo(P->n_classes, nper), r_hi(P->n_classes, 0);
-  for (int r = 0; r < nper; r++) {
-    r_lo[rank_cls[r]] = std::min(r_lo[rank_cls[r]], r);
-    r_hi[rank_cls[r]] = std::max(r_hi[rank_cls[r]], r + 1);
+    R.lo[c] = nper;
+    R.fixed[c] = (float)(2 * ((ci.A * ci.A + ci.L - 1) / ci.L));
   }
-  // split-row stride residue per item: the residue that minimises the
-  // modelled stage cost of its largest run (pieces of period P pair P / 2 taps
-  // per row when P is even; choosing for the largest run alone comes within
-  // 1 % of minimising over all of an item's runs on the benchmark workloads)
-  std::vector<int> rank_residue(nper, -1);
   for (int r = 0; r < nper; r++) {
-    const int Pr = periods[r], SW = degrid_subwarp(P->cls[rank_cls[r]].pmax);
-    if (Pr & 1) continue;
+    const int c = rank_cls[r];
+    const ClassInfo& ci = P->cls[c];
+    R.rec[r] = (float)((periods[r] * periods[r] + ci.L - 1) / ci.L + 1);
+    R.per_cta[r] = (double)R.rec[r] / ci.G;
+    R.period[r] = (int16_t)periods[r];
+    R.lo[c] = std::min(R.lo[c], r);
+    R.hi[c] = std::max(R.hi[c], r + 1);
+    // split-row stride residue: the one that minimises the modelled stage cost
+    // of pieces of this period (they pair P / 2 taps per row when P is even); an
+    // item takes that of its largest run, which comes within 1 % of minimising
+    // over all of its runs on the benchmark workloads
+    R.residue[r] = -1;
+    const int SW = degrid_subwarp(ci.pmax);
     double bc = 0;
-    for (int m = 0; m < 16; m++) {
-      const double c = split_stage_cost(Pr / 2, m, SW);
-      if (rank_residue[r] < 0 || c < bc) {
-        rank_residue[r] = m;
-        bc = c;
+    for (int m = 0; m < 16 && !(periods[r] & 1); m++) {
+      const double c2 = split_stage_cost(periods[r] / 2, m, SW);
+      if (R.residue[r] < 0 || c2 < bc) {
+        R.residue[r] = (int8_t)m;
+        bc = c2;
       }
     }
   }
-  // items of tiles [t0, t1) in tile order, into out
-  auto build_items = [&](int64_t t0, int64_t t1, std::vector<HostItem>& out, int64_t& used) {
-    int64_t top_taps = 0;
-    int top_rank = -1;
-    auto close_item = [&](HostItem& h) {
-      h.it.cls = item_cls_with_residue(h.it.cls, top_rank < 0 ? -1 : rank_residue[top_rank]);
-      top_taps = 0;
-      top_rank = -1;
-      out.push_back(h);
-    };
-    for (int64_t tile = t0; tile < t1; tile++) {
-      const int64_t k0 = tile * nper;
-      if (offs[k0 + nper] == offs[k0]) continue;
-      used++;
-      const int16_t tx = (int16_t)(tile % P->ntx), ty = (int16_t)(tile / P->ntx);
-      for (int c = 0; c < P->n_classes; c++) {
-        if (r_lo[c] >= r_hi[c] || offs[k0 + r_hi[c]] == offs[k0 + r_lo[c]]) continue;
-        const double fixed = fixed_cost(c), cmax = std::max(4.0 * fixed, tau);
-        HostItem cur{};
-        bool open = false;
-        for (int r = r_lo[c]; r < r_hi[c]; r++) {
-          int32_t pos = offs[k0 + r];
-          const int32_t end = offs[k0 + r + 1];
-          const double rcst = rec_cost[r];
-          while (pos < end) {
-            if (!open) {
-              cur.it.start = pos;
-              cur.it.count = 0;
-              cur.it.tile_x = tx;
-              cur.it.tile_y = ty;
-              cur.it.pmax = 0;
-              cur.it.cls = (int16_t)c;
-              cur.cost = fixed;
-              open = true;
-            }
-            int64_t room = (int64_t)((cmax - cur.cost) / rcst);
-            if (room < 1) room = 1;
-            const int32_t take = (int32_t)std::min<int64_t>(room, end - pos);
-            cur.it.count += take;
-            cur.it.pmax = (int16_t)std::max<int>(cur.it.pmax, periods[r]);
-            cur.cost += take * rcst;
-            if ((int64_t)take * periods[r] * periods[r] > top_taps) {
-              top_taps = (int64_t)take * periods[r] * periods[r];
-              top_rank = r;
-            }
-            pos += take;
-            if (cur.cost >= cmax) {
-              close_item(cur);
-              open = false;
-            }
-          }
-        }
-        if (open) close_item(cur);
-      }
-    }
-  };
-  // tiles in contiguous chunks on up to eight host threads, concatenated in
-  // tile order (the same items as one thread makes)
-  const int64_t ntiles = (int64_t)P->ntx * P->nty;
-  const int nth = (int)std::clamp<int64_t>(ntiles / 8192, 1,
-                                           std::min(8u, std::max(1u, std::thread::hardware_concurrency())));
-  std::vector<std::vector<HostItem>> parts(nth);
-  std::vector<int64_t> used(nth, 0);
-  {
-    std::vector<std::thread> pool;
-    for (int i = 1; i < nth; i++) {
-      try {
-        pool.emplace_back(build_items, ntiles * i / nth, ntiles * (i + 1) / nth, std::ref(parts[i]),
-                          std::ref(used[i]));
-      } catch (...) {  // no thread: this one does that chunk below
-        break;
-      }
-    }
-    build_items(0, ntiles / nth, parts[0], used[0]);
-    for (auto& t : pool) t.join();
-    for (int i = (int)pool.size() + 1; i < nth; i++)
-      build_items(ntiles * i / nth, ntiles * (i + 1) / nth, parts[i], used[i]);
-  }
-  std::vector<HostItem> items;
-  int64_t tiles_used = 0;
-  {
-    size_t total = 0;
-    for (auto& v : parts) total += v.size();
-    items.reserve(total);
-    for (int i = 0; i < nth; i++) {
-      items.insert(items.end(), parts[i].begin(), parts[i].end());
-      tiles_used += used[i];
-    }
-  }
-  P->tiles_used = tiles_used;
-  for (auto& h : items) h.grid = 0;
-  std::vector<Item> it_sorted;
-  std::vector<Bundle> bvec;
-  // a batch member's work goes into the batch's own tables instead
-  if (P->own_work) make_bundles(items, P->cls, P->n_classes, it_sorted, bvec);
-  P->n_items = (int)it_sorted.size();
-  P->n_bundles = (int)bvec.size();
-  // the items with their costs (any order), for batched launches
-  P->host_items = std::move(items);
-
-  // ---- fill
-  if ((rc = dalloc(&P->d_recs, P->n_recs)) || (rc = dalloc(&P->d_items, P->n_items)) ||
-      (rc = dalloc(&P->d_bundles, P->n_bundles)))
-    return rc;
-  GB_CUDA_TRY(cudaMemcpyAsync(d_offs, offs.data(), sizeof(int32_t) * (nkeys + 1),
-                              cudaMemcpyHostToDevice, s));
-  GB_CUDA_TRY(cudaMemsetAsync(d_hist, 0, sizeof(int32_t) * nkeys, s));  // reused as cursor
-  std::vector<int32_t> voffs(nvkeys);
-  {
-    int64_t a = 0;
-    for (int64_t k = 0; k < nvkeys; k++) {
-      voffs[k] = (int32_t)a;
-      a += vhist[k];
-    }
-  }
-  GB_CUDA_TRY(cudaMemcpyAsync(d_voffs, voffs.data(), sizeof(int32_t) * nvkeys,
-                              cudaMemcpyHostToDevice, s));
-  GB_CUDA_TRY(cudaMemsetAsync(d_vhist, 0, sizeof(int32_t) * nvkeys, s));  // reused as cursor
-  if (P->n_items)
-    GB_CUDA_TRY(cudaMemcpyAsync(P->d_items, it_sorted.data(), sizeof(Item) * P->n_items,
-                                cudaMemcpyHostToDevice, s));
-  if (P->n_bundles)
-    GB_CUDA_TRY(cudaMemcpyAsync(P->d_bundles, bvec.data(), sizeof(Bundle) * P->n_bundles,
-                                cudaMemcpyHostToDevice, s));
-  if (n_vis > 0) {
-    k_plan_fill<<<blocks_for(n_vis, 256), 256, 0, s>>>(D, P->d_planes, P->T, P->ntx, nper, d_offs,
-                                                       d_hist, P->d_recs, d_voffs, d_vhist,
-                                                       P->d_order);
-    GB_CUDA_TRY(cudaGetLastError());
-  }
+  R.pieces = (double)P->bpc * std::max(1, sm_count() * std::max(1, P->ctas_per_sm_grid));
+  const int iblocks = (int)((nci + 127) / 128);
+  k_plan_items<<<iblocks, 128, 0, s>>>(R, ntiles, P->ntx, d_offs, d_cnt, d_icount, nullptr, nullptr,
+                                       nullptr);
+  GB_CUDA_TRY(cudaGetLastError());
+  if ((rc = scan_keys(d_icount, nci, d_ifirst, d_sums, s))) return rc;
+  k_plan_classes<<<1, 32, 0, s>>>(d_ifirst, ntiles, P->n_classes, d_cnt);
+  GB_CUDA_TRY(cudaGetLastError());
+  PlanCounts cnt;
+  GB_CUDA_TRY(cudaMemcpyAsync(&cnt, d_cnt, sizeof(cnt), cudaMemcpyDeviceToHost, s));
   GB_CUDA_TRY(cudaStreamSynchronize(s));
+  P->kept = (int64_t)cnt.kept;
+  P->taps = (int64_t)cnt.taps;
+  P->n_recs = (int64_t)cnt.recs;
+  P->taps_paired = (int64_t)cnt.paired;
+  P->tiles_used = (int64_t)cnt.tiles;
+  if (P->n_recs >= (int64_t)INT32_MAX) {
+    gb_set_error(GB_ERR_CAPACITY, "more than 2^31 footprint pieces");
+    return GB_ERR_CAPACITY;
+  }
+  const int n_items = cnt.class_first[P->n_classes];
+  P->class_items.clear();
+  for (int c = 0; c < P->n_classes; c++)
+    P->class_items.push_back(cnt.class_first[c + 1] - cnt.class_first[c]);
+
+  // ---- records and items
+  // (the raw costs lie behind the raw items, the bundles behind the items)
+  unsigned char* raw = nullptr;
+  if ((rc = dalloc(&P->d_recs, P->n_recs)) ||
+      (rc = dalloc(&raw, (sizeof(Item) + sizeof(float)) * n_items)))
+    return rc;
+  P->d_raw_items = (Item*)raw;
+  P->d_raw_cost = (float*)(P->d_raw_items + n_items);
+  GB_CUDA_TRY(cudaMemsetAsync(d_hist, 0, sizeof(int32_t) * all, s));  // reused as cursors
+  if (n_vis > 0)
+    k_plan_fill<<<blocks_for(n_vis, 256), 256, 0, s>>>(D, P->d_planes, d_cells, P->T, P->ntx, nper,
+                                                       d_offs, d_hist, P->d_recs, d_offs + nkeys,
+                                                       d_vhist, P->d_order);
+  k_plan_items<<<iblocks, 128, 0, s>>>(R, ntiles, P->ntx, d_offs, d_cnt, nullptr, d_ifirst,
+                                       P->d_raw_items, P->d_raw_cost);
+  GB_CUDA_TRY(cudaGetLastError());
+  // a batch member's items go into the batch's own tables instead
+  P->n_items = n_items;
+  if (P->own_work) {
+    P->n_bundles = count_bundles(P->class_items, P->cls, 1);
+    unsigned char* work = nullptr;
+    if ((rc = dalloc(&work, sizeof(Item) * n_items + sizeof(Bundle) * P->n_bundles))) return rc;
+    P->d_items = (Item*)work;
+    P->d_bundles = (Bundle*)(P->d_items + n_items);
+    if ((rc = bundle_items(P->d_raw_items, P->d_raw_cost, nullptr, n_items, P->class_items, P->cls,
+                           1, P->d_items, P->d_bundles, s)))
+      return rc;
+    P->release_raw();
+  } else {
+    GB_CUDA_TRY(cudaStreamSynchronize(s));
+  }
   return GB_OK;
 }
 

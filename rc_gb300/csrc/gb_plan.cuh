@@ -67,13 +67,6 @@ struct __align__(16) Bundle {
 };
 static_assert(sizeof(Bundle) == 16, "Bundle must be 16 bytes");
 
-// Item with its modelled cost and grid slot, kept on the host to form bundles.
-struct HostItem {
-  Item it;
-  double cost;
-  int grid;
-};
-
 // One thread-group class: L threads per group, G groups per CTA, region edge A.
 struct ClassInfo {
   int32_t L, G, A, pmax;
@@ -185,7 +178,9 @@ struct gb_plan {
   size_t smem_grid = 0, smem_degrid = 0;
   int ctas_per_sm_grid = 1;
   int ctas_per_sm_degrid[3] = {1, 1, 1};  // per GB_STAGE_* form
-  // device arrays owned by the plan
+  // device arrays owned by the plan: one allocation for the tables, one for the
+  // records, one for the items with the bundles behind them
+  unsigned char* d_tables = nullptr;
   int32_t* d_plane = nullptr;
   int32_t* d_order = nullptr;
   int32_t* d_supports = nullptr;
@@ -203,7 +198,12 @@ struct gb_plan {
   int stage_pref = -1;      // GB_STAGE_*: forced staging form of degridding, or -1
   bool own_work = true;     // false for a batch member: no launch tables of its own
   bool own_plane = true;
-  std::vector<gb::HostItem> host_items;  // every item with its cost (grid slot 0)
+  std::vector<int> class_items;  // items per thread-group class
+  // the items by class and their modelled costs, until they are bundled (by the
+  // plan itself, or by the batch of which it is a member)
+  gb::Item* d_raw_items = nullptr;
+  float* d_raw_cost = nullptr;
+  void release_raw();
   // TMA descriptors of the last degridded grid, one per thread-group class
   // (box = that class's stage); rebuilt when the grid's address or shape changes
   const void* tma_grid = nullptr;
@@ -216,11 +216,15 @@ struct gb_plan {
 };
 
 namespace gb {
-// Bundles from items: grouped by (class, grid), by decreasing cost, up to
+// Bundles of n device items: grouped by (class, grid), by decreasing cost, up to
 // cls[c].G items each; all bundles then by decreasing cost (longest first).
-// it_out receives the items in bundle order.
-void make_bundles(const std::vector<HostItem>& items, const ClassInfo* cls, int n_classes,
-                  std::vector<Item>& it_out, std::vector<Bundle>& b_out);
+// grids: each item's grid slot (device), or NULL for one grid; counts: items per
+// (class, grid), grid-fastest.  out receives the items in bundle order, bundles
+// the count_bundles() bundles.  Synchronises the stream.
+int count_bundles(const std::vector<int>& counts, const ClassInfo* cls, int ngrid);
+int bundle_items(const Item* items, const float* cost, const int16_t* grids, int n,
+                 const std::vector<int>& counts, const ClassInfo* cls, int ngrid, Item* out,
+                 Bundle* bundles, cudaStream_t s);
 int launch_grid_plain64(const gb_plan* plan, const double* vis, const double* gcf, double* grid,
                         cudaStream_t s);
 int launch_degrid_plain64(const gb_plan* plan, const double* gcf, const double* grid,
