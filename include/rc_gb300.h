@@ -410,8 +410,8 @@ int gb_batch_degrid_f64(gb_batch *batch, const double *d_gcf, const double *cons
  * return GB_ERR_CAPACITY before any GPU work.  A grid more than 32767 tiles
  * wide or high returns GB_ERR_ARG, as gb_plan_create does.
  *
- * The call synchronises `stream` once (to size the kernel launch), so it
- * cannot be captured into a CUDA graph.  The first call on a device looks up
+ * The call only queues work on `stream` (every input stays in use until that
+ * work is done) and does not synchronise.  The first call on a device looks up
  * the array's device address (cudaGetSymbolAddress) and keeps it for the
  * process: after cudaDeviceReset on a device, do not call this entry point
  * there again.

@@ -7,8 +7,8 @@
 // not touch the allocator for other reasons.  This entry point serves them:
 // it grids up to GB_NOALLOC_MAX_VIS visibilities into the caller's grid with
 // the same tiled FP32 kernel as gb_grid_f32, but keeps every piece of its
-// working memory (plane table, per-visibility planes, histogram, offsets,
-// records, work items, bundles, queue counter) in one file-scope device array
+// working memory (per-visibility cells, histogram, offsets, records, work items,
+// bundles, queue counter) in one file-scope device array
 // of GB_NOALLOC_SCRATCH_BYTES instead of a plan.  It calls no cudaMalloc,
 // cudaFree or allocating library routine.
 //
@@ -18,7 +18,7 @@
 // cudaGetSymbolAddress (once per device, with that device current) and passes
 // that address to the kernels.  Every call on a device shares the array and
 // finds it as the previous call left it: the counters, histogram and cursors
-// that must start at zero are cleared by each call, and calls whose GPU work
+// that must start at zero are cleared by each call (one memset), and calls whose GPU work
 // overlaps (on different streams, or from different host threads) race on the
 // array and must be serialised by the caller.  The cached address belongs to
 // the device's current context: after cudaDeviceReset on a device this entry
@@ -30,6 +30,15 @@
 // of period, with a group barrier), but a mixed bin splits into more, shorter
 // runs than a plan's would, and the FP32 summation order can change from call
 // to call (results agree to FP32 rounding, not bit for bit).
+//
+// The call is one memset and four launches on the caller's stream, without a
+// synchronisation: the number of bundles stays on the device, where the
+// (persistent) gridding kernel reads it, and the plane table travels as a kernel
+// argument.  Bins are cut into items of at most `cut` pieces, so that the few
+// dense tiles of a core-heavy array do not run on one CTA each while the others
+// wait.  4,560 visibilities on 1024^2 (4 planes, supports 8 to 24): 46 us a call;
+// with a bin per item, a plane upload and a read-back 124 us, of which the
+// gridding kernel 59 us.  Denser calls gain more (855 -> 70 us).
 #include <algorithm>
 #include <mutex>
 
@@ -47,24 +56,35 @@ constexpr int kMaxPieces = GB_NOALLOC_MAX_PIECES;
 constexpr int kMaxBins = GB_NOALLOC_MAX_BINS;
 constexpr int kMaxPlanes = GB_NOALLOC_MAX_PLANES;
 
-// byte layout of the scratch array
-constexpr size_t kOffCounters = 0;  // int32[16]: pieces, items, bundles, queue, overflow
-constexpr size_t kOffPlanes = 256;  // PlaneInfo[kMaxPlanes]
-constexpr size_t kOffPlaneOf = align256(kOffPlanes + sizeof(PlaneInfo) * kMaxPlanes);
-constexpr size_t kOffHist = align256(kOffPlaneOf + 4 * (size_t)kMaxVis);
-constexpr size_t kOffOffs = align256(kOffHist + 4 * (size_t)kMaxBins);
-constexpr size_t kOffCursor = align256(kOffOffs + 4 * ((size_t)kMaxBins + 1));
-constexpr size_t kOffRecs = align256(kOffCursor + 4 * (size_t)kMaxBins);
+constexpr int kMaxItems = kMaxBins + 4096;  // bins are cut: one item each and 4096 more
+
+// byte layout of the scratch array (the cursors follow the histogram's bins in
+// use, so that one memset clears counters, histogram and cursors)
+constexpr size_t kOffCounters = 0;  // int32[16]: pieces, items, bundles, queue
+constexpr size_t kOffHist = 256;
+constexpr size_t kOffOffs = align256(kOffHist + 8 * (size_t)kMaxBins);
+constexpr size_t kOffCells = align256(kOffOffs + 4 * ((size_t)kMaxBins + 1));
+constexpr size_t kOffRecs = align256(kOffCells + 8 * (size_t)kMaxVis);
 constexpr size_t kOffItems = align256(kOffRecs + sizeof(Rec) * (size_t)kMaxPieces);
-constexpr size_t kOffBundles = align256(kOffItems + sizeof(Item) * (size_t)kMaxBins);
-constexpr size_t kScratchBytes = align256(kOffBundles + sizeof(Bundle) * (size_t)kMaxBins);
+constexpr size_t kOffBundles = align256(kOffItems + sizeof(Item) * (size_t)kMaxItems);
+constexpr size_t kScratchBytes = align256(kOffBundles + sizeof(Bundle) * (size_t)kMaxItems);
 static_assert(kScratchBytes <= (size_t)GB_NOALLOC_SCRATCH_BYTES,
               "scratch layout exceeds the documented size");
 
-enum { kCntPieces = 0, kCntItems = 1, kCntBundles = 2, kCntQueue = 3, kCntOverflow = 4 };
+enum { kCntPieces = 0, kCntItems = 1, kCntBundles = 2, kCntQueue = 3 };
+
+struct NaPlanes {  // by value: a kernel argument
+  PlaneInfo p[kMaxPlanes];
+};
+
+// A visibility's corner pixel (below 2^22), plane and phase; xp < 0: not gridded.
+struct NaCell {
+  int32_t xp, yp;  // x | plane << 22, y | phase << 24
+};
 
 struct NaClasses {
   int32_t n, ntiles, ntx;
+  int32_t cut;  // pieces per item, at most
   int32_t G[kMaxClasses], pmax[kMaxClasses];
 };
 
@@ -73,69 +93,81 @@ struct NaClasses {
 static __device__ __align__(256) unsigned char g_noalloc_scratch[GB_NOALLOC_SCRATCH_BYTES];
 
 // per visibility: plane, index, then a histogram of pieces per (class, tile)
-__global__ void k_na_count(PlanDev P, const PlaneInfo* __restrict__ pl,
-                           const int32_t* __restrict__ plane_in, int32_t* __restrict__ plane_out,
-                           int32_t n_planes, double w_lo, double w_hi, int32_t T, NaClasses nc,
+__global__ void k_na_count(PlanDev P, const __grid_constant__ NaPlanes pl,
+                           const int32_t* __restrict__ plane_in, int32_t n_planes, double w_lo,
+                           double w_hi, int32_t T, NaClasses nc, NaCell* __restrict__ cells,
                            int32_t* __restrict__ hist) {
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < P.n_vis;
        t += (int64_t)gridDim.x * blockDim.x) {
     const double* r = P.uvw + t * P.uvw_stride;
-    int32_t p = plane_in ? plane_in[t] : w_plane(r[2], w_lo, w_hi, n_planes);
-    if (p >= n_planes) p = -1;
-    plane_out[t] = p;
-    if (p < 0) continue;
-    const PlaneInfo q = pl[p];
-    const VisIndex ix =
-        vis_index(r[0], r[1], P.scale, P.grid_size, q.S, P.margin, 0, 0, P.ext_x, P.ext_y);
-    if (!ix.keep) continue;
-    for (int oy = 0; oy < q.S; oy += q.P)
-      for (int ox = 0; ox < q.S; ox += q.P) {
-        const int tile = ((ix.y0 + oy) / T) * nc.ntx + (ix.x0 + ox) / T;
-        atomicAdd(&hist[q.rank * nc.ntiles + tile], 1);
+    const int32_t p = plane_in ? plane_in[t] : w_plane(r[2], w_lo, w_hi, n_planes);
+    NaCell cell{-1, 0};
+    if (p >= 0 && p < n_planes) {
+      const PlaneInfo q = pl.p[p];
+      const VisIndex ix =
+          vis_index(r[0], r[1], P.scale, P.grid_size, q.S, P.margin, 0, 0, P.ext_x, P.ext_y);
+      if (ix.keep) {
+        cell = NaCell{ix.x0 | p << 22, ix.y0 | ix.phase << 24};
+        for (int oy = 0; oy < q.S; oy += q.P)
+          for (int ox = 0; ox < q.S; ox += q.P) {
+            const int tile = ((ix.y0 + oy) / T) * nc.ntx + (ix.x0 + ox) / T;
+            atomicAdd(&hist[q.rank * nc.ntiles + tile], 1);
+          }
       }
+    }
+    cells[t] = cell;
   }
 }
 
-// one block: offsets (exclusive scan of the histogram), one work item per
-// non-empty (class, tile) bin, and bundles of up to G items of one class
+// one block: offsets (exclusive scan of the histogram), the work items of each
+// (class, tile) bin, and bundles of up to G items of one class, the classes of
+// the larger footprints first
 __global__ void __launch_bounds__(1024) k_na_tables(const int32_t* __restrict__ hist,
                                                     int32_t nkeys, NaClasses nc,
                                                     int32_t* __restrict__ offs,
                                                     Item* __restrict__ items,
                                                     Bundle* __restrict__ bundles,
                                                     int32_t* __restrict__ counters) {
-  __shared__ int s_r[1024], s_i[1024];
+  __shared__ int s_r[32], s_i[32];
   __shared__ int cls_first[kMaxClasses + 1];
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int chunk = (nkeys + 1023) / 1024;
   const int k0 = min(nkeys, tid * chunk), k1 = min(nkeys, k0 + chunk);
   int rsum = 0, isum = 0;
   for (int k = k0; k < k1; k++) {
     const int h = hist[k];
     rsum += h;
-    isum += h > 0;
+    isum += (h + nc.cut - 1) / nc.cut;
   }
-  s_r[tid] = rsum;
-  s_i[tid] = isum;
+  // exclusive scans of both sums over the block
+  int ri = rsum, ii = isum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, ri, o), b = __shfl_up_sync(0xffffffffu, ii, o);
+    if (lane >= o) {
+      ri += a;
+      ii += b;
+    }
+  }
+  if (lane == 31) {
+    s_r[warp] = ri;
+    s_i[warp] = ii;
+  }
   __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {
-    const int a = tid >= off ? s_r[tid - off] : 0;
-    const int b = tid >= off ? s_i[tid - off] : 0;
-    __syncthreads();
-    s_r[tid] += a;
-    s_i[tid] += b;
-    __syncthreads();
+  int rpre = ri - rsum, ipre = ii - isum;
+  for (int w = 0; w < warp; w++) {
+    rpre += s_r[w];
+    ipre += s_i[w];
   }
-  int rpre = s_r[tid] - rsum, ipre = s_i[tid] - isum;
   for (int k = k0; k < k1; k++) {
-    if (k % nc.ntiles == 0) cls_first[k / nc.ntiles] = ipre;
+    const int c = k / nc.ntiles, tile = k - c * nc.ntiles;
+    if (tile == 0) cls_first[c] = ipre;
     const int h = hist[k];
     offs[k] = rpre;
-    if (h > 0) {
-      const int c = k / nc.ntiles, tile = k - c * nc.ntiles;
+    for (int at = 0; at < h; at += nc.cut) {
       Item it;
-      it.start = rpre;
-      it.count = h;
+      it.start = rpre + at;
+      it.count = min(nc.cut, h - at);
       it.tile_x = (int16_t)(tile % nc.ntx);
       it.tile_y = (int16_t)(tile / nc.ntx);
       it.pmax = (int16_t)nc.pmax[c];
@@ -145,60 +177,47 @@ __global__ void __launch_bounds__(1024) k_na_tables(const int32_t* __restrict__ 
     rpre += h;
   }
   if (tid == 1023) {
-    offs[nkeys] = s_r[1023];
-    counters[kCntPieces] = s_r[1023];
-    counters[kCntItems] = s_i[1023];
-    cls_first[nc.n] = s_i[1023];
+    offs[nkeys] = rpre;
+    counters[kCntPieces] = rpre;
+    counters[kCntItems] = ipre;
+    cls_first[nc.n] = ipre;
   }
   __syncthreads();
-  int nb[kMaxClasses], bs[kMaxClasses + 1];
-  bs[0] = 0;
-  for (int c = 0; c < nc.n; c++) {
-    const int n_c = cls_first[c + 1] - cls_first[c];
-    nb[c] = (n_c + nc.G[c] - 1) / nc.G[c];
-    bs[c + 1] = bs[c] + nb[c];
-  }
-  const int total = bs[nc.n];
-  for (int b = tid; b < total; b += 1024) {
-    int c = 0;
-    while (b >= bs[c + 1]) c++;
-    const int j = b - bs[c];
-    const int n_c = cls_first[c + 1] - cls_first[c];
-    Bundle B;
-    B.first_item = cls_first[c] + j * nc.G[c];
-    B.n_items = (int16_t)min(nc.G[c], n_c - j * nc.G[c]);
-    B.cls = (int16_t)c;
-    B.grid = 0;
-    B.pad = 0;
-    bundles[b] = B;
+  int total = 0;
+  for (int c = nc.n - 1; c >= 0; c--) {
+    const int n_c = cls_first[c + 1] - cls_first[c], G = nc.G[c], nb = (n_c + G - 1) / G;
+    for (int j = tid; j < nb; j += 1024) {
+      Bundle B;
+      B.first_item = cls_first[c] + j * G;
+      B.n_items = (int16_t)min(G, n_c - j * G);
+      B.cls = (int16_t)c;
+      B.grid = 0;
+      B.pad = 0;
+      bundles[total + j] = B;
+    }
+    total += nb;
   }
   if (tid == 0) counters[kCntBundles] = total;
 }
 
-__global__ void k_na_fill(PlanDev P, const PlaneInfo* __restrict__ pl, int32_t T, NaClasses nc,
-                          const int32_t* __restrict__ offs, int32_t* __restrict__ cursor,
-                          Rec* __restrict__ recs, int32_t* __restrict__ counters) {
+__global__ void k_na_fill(PlanDev P, const __grid_constant__ NaPlanes pl, int32_t T, NaClasses nc,
+                          const NaCell* __restrict__ cells, const int32_t* __restrict__ offs,
+                          int32_t* __restrict__ cursor, Rec* __restrict__ recs) {
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < P.n_vis;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t p = P.plane[t];
-    if (p < 0) continue;
-    const PlaneInfo q = pl[p];
-    const double* r = P.uvw + t * P.uvw_stride;
-    const VisIndex ix =
-        vis_index(r[0], r[1], P.scale, P.grid_size, q.S, P.margin, 0, 0, P.ext_x, P.ext_y);
-    if (!ix.keep) continue;
-    const int64_t gbase = q.gcf_off + (int64_t)ix.phase * q.S * q.S;
+    const NaCell cell = cells[t];
+    if (cell.xp < 0) continue;
+    const PlaneInfo q = pl.p[cell.xp >> 22];
+    const int x0 = cell.xp & 0x3FFFFF, y0 = cell.yp & 0xFFFFFF, phase = cell.yp >> 24;
+    const int64_t gbase = q.gcf_off + (int64_t)phase * q.S * q.S;
     for (int oy = 0; oy < q.S; oy += q.P) {
-      const int Y0 = ix.y0 + oy, wy = min(q.P, q.S - oy);
+      const int Y0 = y0 + oy, wy = min(q.P, q.S - oy);
       for (int ox = 0; ox < q.S; ox += q.P) {
-        const int X0 = ix.x0 + ox, wx = min(q.P, q.S - ox);
+        const int X0 = x0 + ox, wx = min(q.P, q.S - ox);
         const int tx = X0 / T, ty = Y0 / T;
         const int key = q.rank * nc.ntiles + ty * nc.ntx + tx;
         const int32_t pos = offs[key] + atomicAdd(&cursor[key], 1);
-        if (pos >= kMaxPieces) {  // cannot happen under the host-side bound; never write past
-          atomicExch(&counters[kCntOverflow], 1);
-          continue;
-        }
+        if (pos >= kMaxPieces) continue;  // cannot happen under the host-side bound
         Rec rc;
         rc.vis = (int32_t)t;
         rc.gcf = (uint32_t)(gbase + (int64_t)oy * q.S + ox);
@@ -286,7 +305,8 @@ extern "C" int gb_grid_f32_noalloc(const gb_geometry* geo, int64_t n_vis, const 
     return GB_ERR_ARG;
   }
   // planes -> pieces, periods, classes (the rules of gb_plan_create)
-  thread_local PlaneInfo pl[kMaxPlanes];
+  NaPlanes planes;
+  PlaneInfo* pl = planes.p;
   int widths[kMaxClasses], nwidth = 0, kmax = 1;
   int64_t gcf_len = 0;
   for (int p = 0; p < geo->n_planes; p++) {
@@ -366,31 +386,30 @@ extern "C" int gb_grid_f32_noalloc(const gb_geometry* geo, int64_t n_vis, const 
     return GB_ERR_CAPACITY;
   }
   nc.ntiles = (int32_t)ntiles;
+  // items of 32 pieces or more, four per SM for larger calls, and never more than
+  // 4096 beyond one per bin
+  const int64_t pieces = n_vis * kmax * kmax;
+  nc.cut = (int32_t)std::max<int64_t>({32, (pieces + 4095) / 4096, pieces / (4 * sm_count())});
 
   unsigned char* base = nullptr;
   int rc = scratch_base(&base);
   if (rc) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   int32_t* counters = (int32_t*)(base + kOffCounters);
-  PlaneInfo* d_pl = (PlaneInfo*)(base + kOffPlanes);
-  int32_t* plane_of = (int32_t*)(base + kOffPlaneOf);
   int32_t* hist = (int32_t*)(base + kOffHist);
+  int32_t* cursor = hist + nkeys;
   int32_t* offs = (int32_t*)(base + kOffOffs);
-  int32_t* cursor = (int32_t*)(base + kOffCursor);
+  NaCell* cells = (NaCell*)(base + kOffCells);
   Rec* recs = (Rec*)(base + kOffRecs);
   Item* items = (Item*)(base + kOffItems);
   Bundle* bundles = (Bundle*)(base + kOffBundles);
 
-  GB_CUDA_TRY(cudaMemcpyAsync(d_pl, pl, sizeof(PlaneInfo) * geo->n_planes,
-                              cudaMemcpyHostToDevice, s));
-  GB_CUDA_TRY(cudaMemsetAsync(counters, 0, 64, s));
-  GB_CUDA_TRY(cudaMemsetAsync(hist, 0, sizeof(int32_t) * nkeys, s));
-  GB_CUDA_TRY(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * nkeys, s));
+  GB_CUDA_TRY(cudaMemsetAsync(counters, 0, kOffHist + 2 * sizeof(int32_t) * nkeys, s));
   PlanDev D;
   D.n_vis = n_vis;
   D.uvw = d_uvw;
   D.uvw_stride = uvw_stride;
-  D.plane = plane_of;
+  D.plane = nullptr;
   D.order = nullptr;
   D.supports = nullptr;
   D.gcf_offsets = nullptr;
@@ -402,24 +421,19 @@ extern "C" int gb_grid_f32_noalloc(const gb_geometry* geo, int64_t n_vis, const 
   D.pitch = geo->pitch;
   const int blocks = (int)std::min<int64_t>((n_vis + 255) / 256 + 1, (int64_t)sm_count() * 8);
   if (n_vis > 0) {
-    k_na_count<<<blocks, 256, 0, s>>>(D, d_pl, d_plane, plane_of, geo->n_planes, geo->w_low,
-                                      geo->w_high, T, nc, hist);
+    k_na_count<<<blocks, 256, 0, s>>>(D, planes, d_plane, geo->n_planes, geo->w_low, geo->w_high,
+                                      T, nc, cells, hist);
     GB_CUDA_TRY(cudaGetLastError());
   }
   k_na_tables<<<1, 1024, 0, s>>>(hist, (int32_t)nkeys, nc, offs, items, bundles, counters);
   GB_CUDA_TRY(cudaGetLastError());
   if (n_vis > 0) {
-    k_na_fill<<<blocks, 256, 0, s>>>(D, d_pl, T, nc, offs, cursor, recs, counters);
+    k_na_fill<<<blocks, 256, 0, s>>>(D, planes, T, nc, cells, offs, cursor, recs);
     GB_CUDA_TRY(cudaGetLastError());
   }
-  int32_t hc[8] = {0};
-  GB_CUDA_TRY(cudaMemcpyAsync(hc, counters, sizeof(hc), cudaMemcpyDeviceToHost, s));
-  GB_CUDA_TRY(cudaStreamSynchronize(s));
-  if (hc[kCntOverflow]) {
-    gb_set_error(GB_ERR_CAPACITY, "gb_grid_f32_noalloc: footprint pieces overflowed the scratch");
-    return GB_ERR_CAPACITY;
-  }
-  return launch_grid_tiled_tables(bundles, hc[kCntBundles], items, recs, counters + kCntQueue, cls,
-                                  nwidth, NT, T, geo->ext_x, geo->ext_y, geo->pitch, smem, d_vis,
-                                  d_gcf, d_grid, TiledBounds{hc[kCntPieces], gcf_len, n_vis}, s);
+  const int64_t most = std::min(pieces, nkeys) + pieces / nc.cut;  // bundles
+  return launch_grid_tiled_tables(bundles, counters + kCntBundles, (int)most, items, recs,
+                                  counters + kCntQueue, cls, nwidth, NT, T, geo->ext_x, geo->ext_y,
+                                  geo->pitch, smem, d_vis, d_gcf, d_grid,
+                                  TiledBounds{kMaxPieces, gcf_len, n_vis}, s);
 }

@@ -246,11 +246,12 @@ int plan_create(const gb_geometry* geo, int64_t n_vis, const double* d_uvw, int6
 struct TiledBounds {
   int64_t n_recs, gcf_len, n_vis;
 };
-int launch_grid_tiled_tables(const Bundle* bundles, int n_bundles, const Item* items,
-                             const Rec* recs, int32_t* queue, const ClassInfo* cls, int n_classes,
-                             int NT, int T, int ext_x, int ext_y, int64_t pitch, size_t smem,
-                             const float* vis, const float* gcf, float* grid,
-                             const TiledBounds& bounds, cudaStream_t s);
+int launch_grid_tiled_tables(const Bundle* bundles, const int32_t* n_bundles, int max_bundles,
+                             const Item* items, const Rec* recs, int32_t* queue,
+                             const ClassInfo* cls, int n_classes, int NT, int T, int ext_x,
+                             int ext_y, int64_t pitch, size_t smem, const float* vis,
+                             const float* gcf, float* grid, const TiledBounds& bounds,
+                             cudaStream_t s);
 int launch_tiled_batch(bool grid_mode, int mode, int NT, size_t smem, int ctas_per_sm,
                        const Bundle* bundles, int n_bundles, const Item* items, const Rec* recs,
                        int32_t* queue, const ClassInfo* cls, int n_classes, int T,

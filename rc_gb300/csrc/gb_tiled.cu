@@ -47,6 +47,7 @@ struct TiledArgs {
   int32_t* queue;
   ClassInfo cls[kMaxClasses];
   int32_t n_bundles;
+  const int32_t* n_bundles_dev;  // where gridding reads n_bundles from, or NULL
   int32_t T;
 #ifdef GB_CHECKED
   int64_t n_recs;   // records in `recs`
@@ -369,11 +370,12 @@ __global__ void __launch_bounds__(NT) k_grid_tiled(const __grid_constant__ Tiled
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int s_b;
   const int tid = threadIdx.x;
+  const int n_bundles = a.n_bundles_dev ? *a.n_bundles_dev : a.n_bundles;
   for (;;) {
     if (tid == 0) s_b = atomicAdd(a.queue, 1);
     __syncthreads();
     const int b = s_b;
-    if (b >= a.n_bundles) break;
+    if (b >= n_bundles) break;
     const Bundle bd = a.bundles[b];
     const ClassInfo ci = class_of(a, bd.cls);
     const int g = tid / ci.L;
@@ -860,6 +862,7 @@ static TiledArgs make_args(const gb_plan* P) {
   a.queue = P->d_queue;
   for (int c = 0; c < kMaxClasses; c++) a.cls[c] = P->cls[c];
   a.n_bundles = P->n_bundles;
+  a.n_bundles_dev = nullptr;
   a.T = P->T;
   set_bounds(a, TiledBounds{P->n_recs, P->gcf_len, P->dev.n_vis});
   return a;
@@ -981,30 +984,33 @@ int launch_degrid_tiled(gb_plan* P, const float* gcf, const float* grid, float* 
 }
 
 // Launch of the tiled gridding kernel on caller-supplied work tables (used by
-// the allocation-free entry point, whose tables live in a static device
-// array rather than in a plan).
-int launch_grid_tiled_tables(const Bundle* bundles, int n_bundles, const Item* items,
-                             const Rec* recs, int32_t* queue, const ClassInfo* cls, int n_classes,
-                             int NT, int T, int ext_x, int ext_y, int64_t pitch, size_t smem,
-                             const float* vis, const float* gcf, float* grid,
-                             const TiledBounds& bounds, cudaStream_t s) {
-  if (n_bundles <= 0) return GB_OK;
+// the allocation-free entry point, whose tables live in a static device array
+// rather than in a plan).  The number of bundles is on the device, at most
+// max_bundles; the queue word is zero in stream order.
+int launch_grid_tiled_tables(const Bundle* bundles, const int32_t* n_bundles, int max_bundles,
+                             const Item* items, const Rec* recs, int32_t* queue,
+                             const ClassInfo* cls, int n_classes, int NT, int T, int ext_x,
+                             int ext_y, int64_t pitch, size_t smem, const float* vis,
+                             const float* gcf, float* grid, const TiledBounds& bounds,
+                             cudaStream_t s) {
+  if (max_bundles <= 0) return GB_OK;
   GridFn fn = grid_fn(NT);
   int rc = set_smem_attr((const void*)fn);
   if (rc) return rc;
-  int per_sm = 0;
-  GB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, NT, smem));
-  const int blocks = std::min(n_bundles, sm_count() * std::max(1, per_sm));
+  // CTAs that shared memory lets an SM hold, eight at most: the kernel pulls its
+  // work, so that one too many only finds the queue empty
+  const int per_sm = std::clamp((int)((size_t)tiled_max_smem() / (smem + 1024)), 1, 8);
+  const int blocks = std::min(max_bundles, sm_count() * per_sm);
   TiledArgs a;
   a.bundles = bundles;
   a.items = items;
   a.recs = recs;
   a.queue = queue;
   for (int c = 0; c < kMaxClasses; c++) a.cls[c] = c < n_classes ? cls[c] : ClassInfo{64, 1, 1, 1};
-  a.n_bundles = n_bundles;
+  a.n_bundles = 0;
+  a.n_bundles_dev = n_bundles;
   a.T = T;
   set_bounds(a, bounds);
-  GB_CUDA_TRY(cudaMemsetAsync(queue, 0, sizeof(int32_t), s));
   fn<<<blocks, NT, smem, s>>>(a, one_grid(grid, vis, ext_x, ext_y, pitch, bounds.n_vis),
                               (const float2*)gcf);
   GB_CUDA_TRY(cudaGetLastError());
@@ -1025,6 +1031,7 @@ int launch_tiled_batch(bool grid_mode, int mode, int NT, size_t smem, int ctas_p
   a.queue = queue;
   for (int c = 0; c < kMaxClasses; c++) a.cls[c] = c < n_classes ? cls[c] : ClassInfo{64, 1, 1, 1};
   a.n_bundles = n_bundles;
+  a.n_bundles_dev = nullptr;
   a.T = T;
   set_bounds(a, bounds);
   const int blocks = std::min(n_bundles, sm_count() * std::max(1, ctas_per_sm));
