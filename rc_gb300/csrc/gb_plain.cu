@@ -414,15 +414,18 @@ __device__ __forceinline__ int64_t visit(const PlanDev& P, int64_t i) {
   return P.order && i < P.n_vis ? (int64_t)P.order[i] : i;
 }
 
+// pw visibilities per warp (plain_grid_dims), one after the other, a lane per
+// tap.  Bound by the FP64 pipe: 4 DMUL / DFMA per tap at 2 per clock and SM,
+// 2.2 ms for 3.0e8 taps; the atomics add into lines held by L2.
 __global__ void k_grid_plain64(PlanDev P, const double2* __restrict__ vis,
-                               const double2* __restrict__ gcf, double2* __restrict__ grid) {
+                               const double2* __restrict__ gcf, double2* __restrict__ grid, int pw) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t t0 = 32 * (blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5));
-       t0 < P.n_vis; t0 += 32 * warps) {
+  for (int64_t t0 = pw * (blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5));
+       t0 < P.n_vis; t0 += pw * warps) {
     const int64_t t = visit(P, t0 + lane);
     const LaneIndex mine = plane_index(P, t);
-    const int m = (int)min((int64_t)32, P.n_vis - t0);
+    const int m = (int)min((int64_t)pw, P.n_vis - t0);
     for (int j = 0; j < m; j++) {
       const LaneIndex ix = mine.from(j);
       if (!ix.keep) continue;
@@ -442,17 +445,17 @@ __global__ void k_degrid_plain64(PlanDev P, const double2* __restrict__ gcf,
                                  const float4* __restrict__ gcf_df,
                                  const float4* __restrict__ grid_df,
                                  const int* __restrict__ exps, double2* __restrict__ pred,
-                                 int mode) {
+                                 int mode, int pw) {
   const int lane = threadIdx.x & 31;
   const bool df = exps[0] != kExpNonFinite && exps[1] != kExpNonFinite;
   const int kt = df_scale_exp(exps[0]) + df_scale_exp(exps[1]);
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t t0 = 32 * (blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5));
-       t0 < P.n_vis; t0 += 32 * warps) {
-    const bool mine_ok = t0 + lane < P.n_vis;
+  for (int64_t t0 = pw * (blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5));
+       t0 < P.n_vis; t0 += pw * warps) {
+    const int m = (int)min((int64_t)pw, P.n_vis - t0);
+    const bool mine_ok = lane < m;
     const int64_t t = visit(P, t0 + lane);
     const LaneIndex mine = plane_index(P, t);
-    const int m = (int)min((int64_t)32, P.n_vis - t0);
     float4 acc_df = make_float4(0.f, 0.f, 0.f, 0.f);
     double2 acc = make_double2(0.0, 0.0);
     for (int j = 0; j < m; j++) {
@@ -492,13 +495,20 @@ static int single_degrid_dims(int64_t n, int* blocks, int* pw) {
   return 256;
 }
 
-static int plain_grid_dims(int64_t n, int* blocks) {
-  const int64_t warps_needed = (n + 31) / 32;
-  int64_t b = (warps_needed + 7) / 8;
-  const int64_t cap = (int64_t)sm_count() * 8;
-  if (b > cap) b = cap;
-  if (b < 1) b = 1;
-  *blocks = (int)b;
+// Launch shape of the engine's FP64 pair: pw visibilities per warp, 8 warps
+// per block, as many blocks as that takes.  A visibility costs S*S taps and S
+// differs from plane to plane, so a warp's work is uneven, and the FP64 pipe
+// (gridding) or the issue slots (degridding) of an SM are only kept busy to
+// the end if it has several times its resident warps (32 to 40) to hand out:
+// 320 per SM.  At 32 visibilities per warp and 64 resident warps' worth of
+// blocks, 387072 visibilities (supports 8 to 64) left the SMs idle for 24 % of either kernel; pair of passes 4.36
+// ms, with 200 / 400 / 800 / 1600 warps per SM 3.63 / 3.62 / 3.71 / 3.78 ms
+// (the indexing, one visibility per lane, is repeated per warp).
+static int plain_grid_dims(int64_t n, int* blocks, int* pw) {
+  const int64_t target = (int64_t)sm_count() * 320;
+  *pw = (int)std::clamp<int64_t>((n + target - 1) / target, 1, 32);
+  const int64_t warps = (n + *pw - 1) / *pw;
+  *blocks = (int)std::clamp<int64_t>((warps + 7) / 8, 1, 1 << 30);
   return 256;
 }
 
@@ -995,10 +1005,10 @@ void DfScratch::release() {
 
 int launch_grid_plain64(const gb_plan* plan, const double* vis, const double* gcf, double* grid,
                         cudaStream_t s) {
-  int blocks;
-  const int threads = plain_grid_dims(plan->dev.n_vis, &blocks);
+  int blocks, pw;
+  const int threads = plain_grid_dims(plan->dev.n_vis, &blocks, &pw);
   k_grid_plain64<<<blocks, threads, 0, s>>>(plan->dev, (const double2*)vis, (const double2*)gcf,
-                                            (double2*)grid);
+                                            (double2*)grid, pw);
   GB_CUDA_TRY(cudaGetLastError());
   return GB_OK;
 }
@@ -1011,11 +1021,11 @@ int launch_degrid_plain64(const gb_plan* plan, const double* gcf, const double* 
       (rc = df_prepare(grid, D.ext_x, D.ext_y, D.pitch, gcf, plan->gcf_len, scratch.grid,
                        scratch.gcf, scratch.exps, s)))
     return rc;
-  int blocks;
-  const int threads = plain_grid_dims(D.n_vis, &blocks);
+  int blocks, pw;
+  const int threads = plain_grid_dims(D.n_vis, &blocks, &pw);
   k_degrid_plain64<<<blocks, threads, 0, s>>>(D, (const double2*)gcf, (const double2*)grid,
                                               scratch.gcf, scratch.grid, scratch.exps,
-                                              (double2*)pred, mode);
+                                              (double2*)pred, mode, pw);
   GB_CUDA_TRY(cudaGetLastError());
   return GB_OK;
 }
