@@ -485,13 +485,17 @@ __global__ void k_degrid_plain64(PlanDev P, const double2* __restrict__ gcf,
   }
 }
 
-// Launch shape of k_degrid_single64: pw records per warp (32, fewer for a
-// call too small to occupy every SM with 32 warps), 8 warps per block.
-static int single_degrid_dims(int64_t n, int* blocks, int* pw) {
-  const int64_t target = (int64_t)sm_count() * 32;
+// Launch shape of k_degrid_single64: pw records per warp (32, fewer for a call
+// too small to give every SM 128 warps, five times what it holds), 8 warps per
+// block.  98e3 records of S = 16: with 32 / 64 / 128 / 256 / 512 warps per SM
+// 168 / 133 / 127 / 139 / 164 us; at 32 the SMs idle for a third of it, with
+// many short warps the indexing, once a warp, is what grows.
+static int single_degrid_dims(int64_t n, int S, int* blocks, int* pw) {
+  const int64_t target = (int64_t)sm_count() * 128;
   *pw = (int)std::clamp<int64_t>((n + target - 1) / target, 1, 32);
+  if (S <= 8) *pw = (*pw + 3) & ~3;  // taken four at a time
   const int64_t warps = (n + *pw - 1) / *pw;
-  *blocks = (int)std::clamp<int64_t>((warps + 7) / 8, 1, (int64_t)sm_count() * 8);
+  *blocks = (int)std::clamp<int64_t>((warps + 7) / 8, 1, 1 << 30);
   return 256;
 }
 
@@ -811,8 +815,14 @@ __global__ void __launch_bounds__(ScatShape<S>::NT)
   float4* acc = (float4*)smem;
   ScatRec* srec = (ScatRec*)(acc + Z::RA * Z::As);
   const int64_t n_kept = offs[nkeys - 1];  // the records without a kept footprint come last
-  const int64_t c0 = (int64_t)blockIdx.x * ch;
-  if (c0 >= n_kept) return;
+  // Chunks from both ends of the order inwards: its ends are the grid's first
+  // and last rows of blocks, where records are sparse and a chunk flushes the
+  // region for nearly each of them, the middle the dense core.  The long chunks
+  // thus start first (98e3 records, S = 16, 66 a chunk: 166 us in order, 138
+  // so; three or four times the chunks take 157 and 163).
+  const int64_t nch = (n_kept + ch - 1) / ch, cb = blockIdx.x;
+  if (cb >= nch) return;
+  const int64_t c0 = (cb & 1 ? nch - 1 - cb / 2 : cb / 2) * ch;
   const int64_t c1 = min(n_kept, c0 + ch);
   const int t = threadIdx.x;
   if (exps[0] == kExpNonFinite || exps[1] == kExpNonFinite) {
@@ -1266,7 +1276,7 @@ static int compat_degrid(const char* who, int size_err, double scale, int32_t gr
     // one launch over the records in grid-block order (neighbouring warps
     // gather from the same grid lines), then one download of the results
     int blocks, pw;
-    const int threads = single_degrid_dims(n, &blocks, &pw);
+    const int threads = single_degrid_dims(n, S, &blocks, &pw);
     k_degrid_single64<<<blocks, threads, 0, s>>>(
         n, (const double*)d_vis, (const double2*)d_gcf, (const double2*)d_grid,
         (const float4*)d_gcf_df, (const float4*)d_grid_df, d_exps, (double*)d_out, geo, order,
@@ -1288,7 +1298,7 @@ static int compat_degrid(const char* who, int size_err, double scale, int32_t gr
   for (int c = 0; c < chunks; c++) {
     const int64_t c0 = n * c / chunks, c1 = n * (c + 1) / chunks;
     int blocks, pw;
-    const int threads = single_degrid_dims(c1 - c0, &blocks, &pw);
+    const int threads = single_degrid_dims(c1 - c0, S, &blocks, &pw);
     k_degrid_single64<<<blocks, threads, 0, s>>>(
         c1 - c0, (const double*)d_vis + 5 * c0, (const double2*)d_gcf, (const double2*)d_grid,
         (const float4*)d_gcf_df, (const float4*)d_grid_df, d_exps, (double*)d_out + 5 * c0, geo,
