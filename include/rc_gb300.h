@@ -435,7 +435,11 @@ int gb_grid_f32_noalloc(const gb_geometry *geo, int64_t n_vis, const double *d_u
  *   image_to_grid: grid = fftshift(FFT(ifftshift(x / (t_y t_x))))   (exp(-2 pi i))
  *   grid_to_image: x    = Re[fftshift(IFFT(ifftshift(grid))) / (t_y t_x)]
  * with IFFT unnormalised (exp(+2 pi i)), so grid_to_image is the exact adjoint
- * of image_to_grid.  d_work: n*n complex scratch (not aliasing d_grid). */
+ * of image_to_grid.  d_work: n*n complex scratch (not aliasing d_grid).
+ * FP32, even n of 16 .. 8192 without a prime factor above 7: the first call of a
+ * size on a device makes the transform's tables (10 n bytes, kept) and waits for
+ * their copy, also inside a stream capture.  Other sizes and FP64 go through
+ * cuFFT plans, made on a size's first call: make that before any capture. */
 int gb_image_to_grid_f32(const float *d_image, const float *d_taper, int32_t n, float *d_grid,
                          void *stream);
 int gb_grid_to_image_f32(const float *d_grid, const float *d_taper, int32_t n, float *d_work,

@@ -483,6 +483,20 @@ bool factor(int n, FftPlan* p) {
   return true;
 }
 
+// Two host arrays into device memory, there for every stream once this returns: a
+// plain cudaMemcpy from pageable memory may return when the data is staged, and
+// runs on the default stream, which non-blocking streams do not wait for.
+cudaError_t upload(void* d0, const void* h0, size_t n0, void* d1, const void* h1, size_t n1) {
+  cudaStream_t up;
+  cudaError_t e = cudaStreamCreateWithFlags(&up, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return e;
+  e = cudaMemcpyAsync(d0, h0, n0, cudaMemcpyHostToDevice, up);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d1, h1, n1, cudaMemcpyHostToDevice, up);
+  const cudaError_t w = cudaStreamSynchronize(up);  // also where the second copy failed
+  cudaStreamDestroy(up);
+  return e != cudaSuccess ? e : w;
+}
+
 int fft_tables(int n, FftPlan* out) {
   static std::mutex mu;
   static std::map<std::pair<int, int>, FftPlan> plans;
@@ -519,15 +533,20 @@ int fft_tables(int n, FftPlan* out) {
     }
     rev[b] = (uint16_t)f;
   }
+  // A first call may come while a stream of this or another thread is captured:
+  // the allocation and the copy are no part of that.
+  struct Relaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  } relaxed;
   void* d = nullptr;
   const int rc = dev_alloc(&d, sizeof(float2) * n + sizeof(uint16_t) * n, "FFT tables");
   if (rc) return rc;
   p.tw = (const float2*)d;
   p.rev = (const uint16_t*)(p.tw + n);
-  cudaError_t e = cudaMemcpy((void*)p.tw, tw.data(), sizeof(float2) * n, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess)
-    e = cudaMemcpy((void*)p.rev, rev.data(), sizeof(uint16_t) * rev.size(),
-                   cudaMemcpyHostToDevice);
+  const cudaError_t e = upload((void*)p.tw, tw.data(), sizeof(float2) * n, (void*)p.rev, rev.data(),
+                               sizeof(uint16_t) * rev.size());
   if (e != cudaSuccess) {
     cudaFree(d);
     GB_CUDA_TRY(e);
