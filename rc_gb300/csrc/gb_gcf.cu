@@ -85,6 +85,9 @@ __global__ void k_gcf_screen(const GcfPlaneDev* __restrict__ planes, int p0, int
 constexpr int kGcfLines = 8;      // lines that a block transforms together
 constexpr int kGcfThreads = 128;
 constexpr int kGcfStages = 8;
+// A block's shared memory: its lines of M values, before and after a transform.
+constexpr size_t gcf_smem(int M) { return sizeof(double2) * 2 * kGcfLines * (M + 1); }
+constexpr int kGcfSmem = (int)gcf_smem(GB_MAX_SUPPORT);
 
 struct GcfFft {
   int M, N, stages;
@@ -371,9 +374,11 @@ static int gcf_pruned(const std::vector<GcfPlaneDev>& hp, const GcfFft& p, doubl
   GcfPlaneDev* d_planes = (GcfPlaneDev*)d;
   double2* w = (double2*)(d + planes_bytes);
   double2* g = w + p.N;
-  const size_t smem = sizeof(double2) * 2 * kGcfLines * (p.M + 1);
-  GB_CUDA_GOTO(cudaFuncSetAttribute(k_gcf_first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  GB_CUDA_GOTO(cudaFuncSetAttribute(k_gcf_second, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const size_t smem = gcf_smem(p.M);
+  // the limit is the kernels', not this call's: the same for every support, so that
+  // calls of other threads cannot lower it below what this one launches with
+  GB_CUDA_GOTO(cudaFuncSetAttribute(k_gcf_first, cudaFuncAttributeMaxDynamicSharedMemorySize, kGcfSmem));
+  GB_CUDA_GOTO(cudaFuncSetAttribute(k_gcf_second, cudaFuncAttributeMaxDynamicSharedMemorySize, kGcfSmem));
   GB_CUDA_GOTO(cudaMemcpyAsync(d_planes, hp.data(), sizeof(GcfPlaneDev) * n_planes,
                                cudaMemcpyHostToDevice, s));
   k_gcf_roots<<<(p.N + 255) / 256, 256, 0, s>>>(p.N, w);
@@ -409,15 +414,15 @@ extern "C" int gb_gcf_generate(int32_t n_planes, const double* w_planes, const i
     }
   }
   cudaStream_t s = (cudaStream_t)stream;
+  std::vector<GcfPlaneDev> hp(n_planes);
+  for (int p = 0; p < n_planes; p++) hp[p] = GcfPlaneDev{w_planes[p], supports[p], gcf_offsets[p]};
+  GcfFft fft;
+  if (gcf_factor(max_support, &fft)) return gcf_pruned(hp, fft, t2, d_taper, d_gcf64, d_gcf32, s);
   const int N = GB_OVER * max_support;
   const size_t arena_bytes = (size_t)N * N * sizeof(double2);
   // batch so that the FFT arenas stay within ~1 GiB
   int batch = (int)std::max<size_t>(1, ((size_t)1 << 30) / arena_bytes);
   batch = std::min(batch, n_planes);
-  std::vector<GcfPlaneDev> hp(n_planes);
-  for (int p = 0; p < n_planes; p++) hp[p] = GcfPlaneDev{w_planes[p], supports[p], gcf_offsets[p]};
-  GcfFft fft;
-  if (gcf_factor(max_support, &fft)) return gcf_pruned(hp, fft, t2, d_taper, d_gcf64, d_gcf32, s);
   int rc = GB_OK;
   GcfPlaneDev* d_planes = nullptr;
   double2* arena = nullptr;
