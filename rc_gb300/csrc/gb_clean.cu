@@ -598,12 +598,8 @@ extern "C" int gb_hogbom_f32(float* d_residual, int32_t nx, int32_t ny, const fl
   a.gain = gain;
   a.threshold = threshold;
   a.n_iter = n_iter;
-  const int64_t want = (ntx * nty + kCleanOwners - 1) / kCleanOwners;
-  const int grid = (int)std::min<int64_t>({want, (int64_t)sm_count(), (int64_t)kCleanCtas});
-  const int64_t owners = (int64_t)grid * kCleanOwners;
   a.ntx = (int)ntx;
   a.ntiles = (int)(ntx * nty);
-  a.local = (int)((ntx * nty + owners - 1) / owners);
   // A component lies within the image, so only the part of the PSF less than the
   // image's size away from its peak can: of a small image's large PSF a few blocks,
   // not a table that its few CTAs would take milliseconds for (64^2, PSF 4096^2, one
@@ -618,15 +614,28 @@ extern "C" int gb_hogbom_f32(float* d_residual, int32_t nx, int32_t ny, const fl
   a.nbx = (int)blocks(a.wx1 - a.wx0);
   a.nby = (int)blocks(a.wy1 - a.wy0);
   const size_t table = sizeof(float) * (size_t)((a.nbx * a.nby + 3) & ~3);
-  const size_t own = sizeof(CleanTile) * (size_t)a.local * kCleanOwners;
-  a.far_tiles = table + own > kCleanSmem ? (CleanTile*)(a.w + 1) : nullptr;
-  const size_t smem = a.far_tiles ? table : table + own;
   GB_CUDA_TRY(cudaFuncSetAttribute((const void*)k_clean, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)kCleanSmem));
   void* args[] = {&a};
-  GB_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_clean, dim3(grid), dim3(kCleanThreads),
-                                          args, smem, s));
-  return GB_OK;
+  const int64_t want = (ntx * nty + kCleanOwners - 1) / kCleanOwners;
+  // The CTAs wait for one another, so all must fit at once.  A process may have fewer
+  // multiprocessors than the device (a partition of it): a grid that is refused for
+  // that is halved, down to one CTA.
+  for (int grid = (int)std::min<int64_t>({want, (int64_t)sm_count(), (int64_t)kCleanCtas});;
+       grid = (grid + 1) / 2) {
+    const int64_t owners = (int64_t)grid * kCleanOwners;
+    a.local = (int)((ntx * nty + owners - 1) / owners);
+    const size_t own = sizeof(CleanTile) * (size_t)a.local * kCleanOwners;
+    a.far_tiles = table + own > kCleanSmem ? (CleanTile*)(a.w + 1) : nullptr;
+    const cudaError_t e =
+        cudaLaunchCooperativeKernel((const void*)k_clean, dim3(grid), dim3(kCleanThreads), args,
+                                    a.far_tiles ? table : table + own, s);
+    if (e != cudaErrorCooperativeLaunchTooLarge || grid == 1) {
+      GB_CUDA_TRY(e);
+      return GB_OK;
+    }
+    (void)cudaGetLastError();  // not the next call's
+  }
 }
 
 extern "C" int gb_hogbom_work_bytes(int32_t nx, int32_t ny, int64_t* out) {

@@ -58,3 +58,25 @@ def test_psf_table_covers_what_can_lie_on_the_image(fake, nx, ny, pnx, pny, ppx,
         assert w0 == max(0, pp - (n - 1)) and w1 == min(pn, pp + n)
         assert (nb - 1 << a.eb) < w1 - w0 <= nb << a.eb
     assert a.nbx * a.nby <= MAX_BLOCKS and a.eb >= 5
+
+
+@pytest.mark.parametrize("limit", [152, 151, 100, 8, 1])
+@pytest.mark.parametrize("nx,ny", [(2048, 2048), (333, 200), (1, 20_000_000)])
+def test_fewer_multiprocessors_than_the_device_has(fake, limit, nx, ny):
+    """Where a process may use only some of the device's multiprocessors, a
+    cooperative launch of one CTA for each of the device's is refused; a smaller one
+    runs, and its warps hold all tiles."""
+    fake.lib.fake_coop_limit(limit)
+    try:
+        a, ops = _launch(fake, nx, ny, 9, 9, 4, 4)
+    finally:
+        fake.lib.fake_coop_limit(1 << 30)
+    ran = [o for o in ops if o.startswith("coop")]
+    assert len(ran) == 1
+    grid, smem = (int(ran[0].split(f"{k}=")[1].split()[0]) for k in ("grid", "smem"))
+    assert grid <= limit and (grid * 2 >= limit or grid * OWNERS >= a.ntiles)
+    assert a.ntiles == -(-nx // TILE_W) * -(-ny // TILE_H)
+    assert a.local * grid * OWNERS >= a.ntiles > (a.local - 1) * grid * OWNERS
+    table = -(-a.nbx * a.nby // 4) * 16
+    assert smem == table + (0 if a.far else a.local * OWNERS * TILE_BYTES) <= 200 * 1024
+    assert bool(a.far) == (table + a.local * OWNERS * TILE_BYTES > 200 * 1024)
