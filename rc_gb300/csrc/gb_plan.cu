@@ -229,78 +229,125 @@ struct ItemRule {
 // The items of each (class, tile): counted (per class, tile-fastest), or with
 // `items` written from first[] on.  An item is closed when its cost reaches the
 // larger of four times its fixed cost and an even share of all the work.
+// A thread to a (class, tile).  Most are empty or give an item or two, but a core-heavy
+// array puts much of its work into a few tiles, each of thousands of items: those of
+// one period are alike, so they are counted by a division and written by the whole warp.
+// A plan of 1e6 visibilities of support 8, all in one tile: 0.71 ms, with a thread
+// cutting its items one by one 4.7 ms (on host threads 2.5 ms); 8e6: 1.45 ms, 4.9
+// and 11.7; 1e6 of a core-heavy array on 256^2: 0.81 ms, 2.96 and 1.92.
 __global__ void __launch_bounds__(128)
     k_plan_items(const __grid_constant__ ItemRule R, int64_t ntiles, int32_t ntx,
                  const int32_t* __restrict__ offs, PlanCounts* __restrict__ cnt,
                  int32_t* __restrict__ count, const int32_t* __restrict__ first,
                  Item* __restrict__ items, float* __restrict__ costs) {
   __shared__ float s_tau;
+  __shared__ bool s_over;
   if (threadIdx.x == 0) {
     double total = 0;
     for (int r = 0; r < R.nper; r++) total += (double)cnt->rank[r] * R.per_cta[r];
     s_tau = (float)(total / R.pieces);
+    s_over = cnt->recs >= (unsigned long long)INT32_MAX;  // refused by the host: offs wrapped
   }
   __syncthreads();
+  const int lane = threadIdx.x & 31;
   const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int c = (int)(e / ntiles);
-  const int64_t tile = e - c * ntiles;
-  bool used = false;
-  if (c < R.nclass) {
-    const int64_t k0 = tile * R.nper;
-    const int32_t b0 = offs[k0 + R.lo[c]], b1 = offs[k0 + R.hi[c]];
+  const int c = min((int)(e / ntiles), R.nclass - 1);
+  const int64_t tile = e % ntiles;
+  const bool live = e < ntiles * R.nclass;
+  bool used = false, any = false;
+  const int64_t k0 = tile * R.nper;
+  int32_t start = 0;
+  if (live && !s_over) {
+    start = offs[k0 + R.lo[c]];
+    any = start != offs[k0 + R.hi[c]];
     used = c == 0 && offs[k0 + R.nper] != offs[k0];
-    int n = 0;
-    if (b1 != b0) {
-      int64_t at = items ? first[e] : 0;
-      const float fixed = R.fixed[c], cmax = fmaxf(4.f * fixed, s_tau);
-      float cost = fixed;
-      int32_t start = b0, in_item = 0;
-      int64_t top_taps = 0;
-      int top = -1, pmax = 0;
-      auto close = [&]() {
-        if (items) {
-          Item it;
-          it.start = start;
-          it.count = in_item;
-          it.tile_x = (int16_t)(tile % ntx);
-          it.tile_y = (int16_t)(tile / ntx);
-          it.pmax = (int16_t)pmax;
-          it.cls = item_cls_with_residue((int16_t)c, R.residue[top]);
-          items[at] = it;
-          costs[at] = cost;
-          at++;
-        }
-        n++;
-        start += in_item;
-        in_item = 0;
-        cost = fixed;
-        top_taps = 0;
-        pmax = 0;
-      };
-      for (int r = R.lo[c]; r < R.hi[c]; r++) {
-        int32_t pos = offs[k0 + r];
-        const int32_t end = offs[k0 + r + 1];
-        const float rc = R.rec[r], per = 1.f / rc;
-        while (pos < end) {
-          const float room = fminf((cmax - cost) * per, 2e9f);
-          const int32_t take = min(max((int32_t)room, 1), end - pos);
-          const int64_t t = (int64_t)take * R.period[r] * R.period[r];
-          if (t > top_taps) {  // the stage stride goes by the largest run
-            top_taps = t;
-            top = r;
-          }
-          pmax = R.period[r];
-          in_item += take;
-          cost += (float)take * rc;
-          pos += take;
-          if (cost >= cmax) close();
-        }
-      }
-      if (in_item) close();
-    }
-    if (!items) count[e] = n;
   }
+  const float fixed = R.fixed[c], cmax = fmaxf(4.f * fixed, s_tau);
+  int64_t at = items && any ? first[e] : 0;
+  float cost = fixed;
+  int32_t in_item = 0, n = 0;
+  int64_t top_taps = 0;
+  int top = -1, pmax = 0;
+  auto write = [&](int64_t to, int64_t tile_, int c_, int32_t start_, int32_t count_, int pmax_, int top_,
+                   float cost_) {
+    Item it;
+    it.start = start_;
+    it.count = count_;
+    it.tile_x = (int16_t)(tile_ % ntx);
+    it.tile_y = (int16_t)(tile_ / ntx);
+    it.pmax = (int16_t)pmax_;
+    it.cls = item_cls_with_residue((int16_t)c_, R.residue[top_]);
+    items[to] = it;
+    costs[to] = cost_;
+  };
+  auto close = [&]() {
+    if (items) write(at, tile, c, start, in_item, pmax, top, cost);
+    at++;
+    n++;
+    start += in_item;
+    in_item = 0;
+    cost = fixed;
+    top_taps = 0;
+    pmax = 0;
+  };
+  // as many records of rank r as the open item has room for
+  auto step = [&](int r, int32_t& pos, int32_t end) {
+    const float rc = R.rec[r], room = fminf((cmax - cost) * (1.f / rc), 2e9f);
+    const int32_t take = min(max((int32_t)room, 1), end - pos);
+    const int64_t t = (int64_t)take * R.period[r] * R.period[r];
+    if (t > top_taps) {  // the stage stride goes by the largest run
+      top_taps = t;
+      top = r;
+    }
+    pmax = R.period[r];
+    in_item += take;
+    cost += (float)take * rc;
+    pos += take;
+    if (cost >= cmax) close();
+  };
+  const int r0 = __reduce_min_sync(0xffffffffu, any ? R.lo[c] : R.nper);
+  const int r1 = __reduce_max_sync(0xffffffffu, any ? R.hi[c] : 0);
+  for (int r = r0; r < r1; r++) {
+    int32_t pos = 0, end = 0, whole = 0, per = 0;
+    float per_cost = fixed;
+    if (any && r >= R.lo[c] && r < R.hi[c]) {
+      pos = offs[k0 + r];
+      end = offs[k0 + r + 1];
+      while (in_item && pos < end) step(r, pos, end);
+      if (pos < end) {  // the records of an item of this rank alone, step by step
+        const float rc = R.rec[r];
+        while (per_cost < cmax && per < end - pos) {
+          const float room = fminf((cmax - per_cost) * (1.f / rc), 2e9f);
+          const int32_t take = min(max((int32_t)room, 1), end - pos - per);
+          per_cost += (float)take * rc;
+          per += take;
+        }
+        if (per_cost >= cmax) whole = (end - pos) / per;
+      }
+    }
+    if (items) {
+      for (unsigned many = __ballot_sync(0xffffffffu, whole >= 32); many; many &= many - 1) {
+        const int src = __ffs(many) - 1;
+        const int64_t to = __shfl_sync(0xffffffffu, at, src), tl = __shfl_sync(0xffffffffu, tile, src);
+        const int cl = __shfl_sync(0xffffffffu, c, src), m = __shfl_sync(0xffffffffu, whole, src);
+        const int32_t p = __shfl_sync(0xffffffffu, per, src), s0 = __shfl_sync(0xffffffffu, pos, src);
+        const float pc = __shfl_sync(0xffffffffu, per_cost, src);
+        for (int i = lane; i < m; i += 32) write(to + i, tl, cl, s0 + i * p, p, R.period[r], r, pc);
+      }
+      if (whole < 32)
+        for (int i = 0; i < whole; i++) write(at + i, tile, c, pos + i * per, per, R.period[r], r, per_cost);
+    }
+    if (whole) {
+      at += whole;
+      n += whole;
+      pos += whole * per;
+      start = pos;
+    }
+    while (pos < end) step(r, pos, end);
+  }
+  if (in_item) close();
   if (!items) {
+    if (live) count[e] = n;
     const int used_here = __syncthreads_count(used);
     if (threadIdx.x == 0 && used_here) atomicAdd(&cnt->tiles, (unsigned long long)used_here);
   }
