@@ -417,12 +417,23 @@ __device__ __forceinline__ int64_t visit(const PlanDev& P, int64_t i) {
 // pw visibilities per warp (plain_grid_dims), one after the other, a lane per
 // tap.  Bound by the FP64 pipe: 4 DMUL / DFMA per tap at 2 per clock and SM,
 // 2.2 ms for 3.0e8 taps; the atomics add into lines held by L2.
+// The visit order brings neighbours on the grid together, so that blocks that run at
+// the same time would all add to the dense core's pixels, one after the other.  They
+// take their shares from kSpread places of the order instead.  8e6 visibilities of
+// support 8, core-heavy: in order 12.0 ms, from 8 / 64 / 512 places 7.8 / 5.4 / 5.3;
+// spread evenly over the grid 4.2 all; 256 antennas, 4.18e6, supports 8 to 64: in order
+// 14.3 ms, 12.6 / 12.1 / 12.0.
+constexpr int kSpread = 512;
+
 __global__ void k_grid_plain64(PlanDev P, const double2* __restrict__ vis,
                                const double2* __restrict__ gcf, double2* __restrict__ grid, int pw) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t t0 = pw * (blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5));
-       t0 < P.n_vis; t0 += pw * warps) {
+  const int64_t per = gridDim.x / kSpread;  // blocks of a part
+  const int64_t b = blockIdx.x < per * kSpread ? blockIdx.x % kSpread * per + blockIdx.x / kSpread
+                                               : blockIdx.x;
+  for (int64_t t0 = pw * (b * (blockDim.x >> 5) + (threadIdx.x >> 5)); t0 < P.n_vis;
+       t0 += pw * warps) {
     const int64_t t = visit(P, t0 + lane);
     const LaneIndex mine = plane_index(P, t);
     const int m = (int)min((int64_t)pw, P.n_vis - t0);
@@ -503,14 +514,22 @@ static int single_degrid_dims(int64_t n, int S, int* blocks, int* pw) {
 // per block, as many blocks as that takes.  A visibility costs S*S taps and S
 // differs from plane to plane, so a warp's work is uneven, and the FP64 pipe
 // (gridding) or the issue slots (degridding) of an SM are only kept busy to
-// the end if it has several times its resident warps (32 to 40) to hand out:
-// 320 per SM.  At 32 visibilities per warp and 64 resident warps' worth of
-// blocks, 387072 visibilities (supports 8 to 64) left the SMs idle for 24 % of either kernel; pair of passes 4.36
-// ms, with 200 / 400 / 800 / 1600 warps per SM 3.63 / 3.62 / 3.71 / 3.78 ms
-// (the indexing, one visibility per lane, is repeated per warp).
-static int plain_grid_dims(int64_t n, int* blocks, int* pw) {
-  const int64_t target = (int64_t)sm_count() * 320;
-  *pw = (int)std::clamp<int64_t>((n + target - 1) / target, 1, 32);
+// the end if it has several times its resident warps (32 to 40) to hand out: 320
+// per SM.  387,072 visibilities (supports 8 to 64), grid and degrid in us: at 32
+// visibilities per warp 2826 and 1355, with 64 / 320 warps per SM 2786 / 2336 and
+// 1259 / 1105.  But the indexing, one visibility per lane, is repeated per warp, and
+// small footprints (the largest support says it) are too little work for that:
+//   supports to 8: at least 8 per warp, and 32 (grid) or 64 (degrid) warps per SM.
+//     129,024 of support 8: at 320 per SM 150 and 198 us, at 64 98 and 149; 65,000 of
+//     support 4: at 320 85 and 166, at 64 47 and 115, at 32 42 and 111;
+//   supports to 24: 64 and 128.  65,000 of support 16: at 320 194 and 180 us, at 128 172
+//     and 160, at 64 160 and 155; 520,000: 1061, 1022, 1053 and 527, 527, 543.
+//   Supports to 32, 65,000: at 320 557 and 290, at 64 541 and 289 us; to 48: 1161 and
+//     498, 1173 and 519.
+static int plain_grid_dims(int64_t n, int max_support, bool grid, int* blocks, int* pw) {
+  const int per_sm = max_support <= 8 ? (grid ? 32 : 64) : max_support <= 24 ? (grid ? 64 : 128) : 320;
+  const int64_t target = (int64_t)sm_count() * per_sm;
+  *pw = (int)std::clamp<int64_t>((n + target - 1) / target, max_support <= 8 ? 8 : 1, 32);
   const int64_t warps = (n + *pw - 1) / *pw;
   *blocks = (int)std::clamp<int64_t>((warps + 7) / 8, 1, 1 << 30);
   return 256;
@@ -1016,7 +1035,7 @@ void DfScratch::release() {
 int launch_grid_plain64(const gb_plan* plan, const double* vis, const double* gcf, double* grid,
                         cudaStream_t s) {
   int blocks, pw;
-  const int threads = plain_grid_dims(plan->dev.n_vis, &blocks, &pw);
+  const int threads = plain_grid_dims(plan->dev.n_vis, plan->max_support, true, &blocks, &pw);
   k_grid_plain64<<<blocks, threads, 0, s>>>(plan->dev, (const double2*)vis, (const double2*)gcf,
                                             (double2*)grid, pw);
   GB_CUDA_TRY(cudaGetLastError());
@@ -1032,7 +1051,7 @@ int launch_degrid_plain64(const gb_plan* plan, const double* gcf, const double* 
                        scratch.gcf, scratch.exps, s)))
     return rc;
   int blocks, pw;
-  const int threads = plain_grid_dims(D.n_vis, &blocks, &pw);
+  const int threads = plain_grid_dims(D.n_vis, plan->max_support, false, &blocks, &pw);
   k_degrid_plain64<<<blocks, threads, 0, s>>>(D, (const double2*)gcf, (const double2*)grid,
                                               scratch.gcf, scratch.grid, scratch.exps,
                                               (double2*)pred, mode, pw);
