@@ -568,9 +568,11 @@ constexpr int kBlk = 32;
 // footprint overlaps; with `exp`, *exp max-ed with the largest exponent field of
 // the visibilities (k_max_exponent's rule).  A warp's records mostly share a
 // few keys (neighbouring samples of a baseline): one atomic per key and warp.
-// On 100,000 records over a 1024^2 grid this takes 23 to 41 us and the scatter
-// below 7 us; with marks, exponent, histogram and scatter as kernels of their own,
-// an atomic per record or warp, they took 15, 129, 35 and 33 us.
+// On 100,000 records over a 1024^2 grid this takes 16 us and the scatter 11 to 12;
+// over 4096^2 13 and 4, a dense core there 30 and 8.  (A mark is stored, not read
+// first: the reads are a chain, 42 us and over 4096^2 67 of them.)  With marks, exponent,
+// histogram and scatter as kernels of their own, an atomic per record or warp, they took
+// 15, 129, 35 and 33 us on the records of a real array.
 __global__ void __launch_bounds__(256) k_record_keys(int64_t n, const double* __restrict__ vis5,
                                                      SingleGeo geo, int nbx, int nkeys,
                                                      unsigned char* __restrict__ marks,
@@ -591,7 +593,7 @@ __global__ void __launch_bounds__(256) k_record_keys(int64_t n, const double* __
         const int bx1 = (x0 + geo.S - 1) / kBlk, by1 = (y0 + geo.S - 1) / kBlk;
         for (int by = y0 / kBlk; by <= by1; by++)
           for (int bx = x0 / kBlk; bx <= bx1; bx++)
-            if (!marks[by * nbx + bx]) marks[by * nbx + bx] = 1;
+            marks[by * nbx + bx] = 1;
       }
     }
     keys[t] = key;
