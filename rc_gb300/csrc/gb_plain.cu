@@ -500,10 +500,13 @@ __global__ void k_degrid_plain64(PlanDev P, const double2* __restrict__ gcf,
 // too small to give every SM 128 warps, five times what it holds), 8 warps per
 // block.  98e3 records of S = 16: with 32 / 64 / 128 / 256 / 512 warps per SM
 // 168 / 133 / 127 / 139 / 164 us; at 32 the SMs idle for a third of it, with
-// many short warps the indexing, once a warp, is what grows.
+// many short warps the indexing, once a warp, is what grows.  So S to 16 has four to a
+// warp as long as every SM still gets eight warps: a call of 10,000 of S = 16 (256^2
+// grid) takes 127 us, with one to a warp 139; of 1,000 161, with four 171.
 static int single_degrid_dims(int64_t n, int S, int* blocks, int* pw) {
   const int64_t target = (int64_t)sm_count() * 128;
-  *pw = (int)std::clamp<int64_t>((n + target - 1) / target, 1, 32);
+  const int64_t least = S <= 16 ? std::clamp<int64_t>(n / (sm_count() * 8), 1, 4) : 1;
+  *pw = (int)std::clamp<int64_t>((n + target - 1) / target, least, 32);
   if (S <= 8) *pw = (*pw + 3) & ~3;  // taken four at a time
   const int64_t warps = (n + *pw - 1) / *pw;
   *blocks = (int)std::clamp<int64_t>((warps + 7) / 8, 1, 1 << 30);
