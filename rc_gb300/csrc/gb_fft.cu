@@ -26,11 +26,14 @@
 // both ways: 60 to 76).  Both directions at 4096^2 take 246 us, rows 45 to 55 us
 // and columns 67 to 74 us (floor at the copy bandwidth: 59 us for both
 // directions; with cuFFT 541 us); 2048^2 84 us (with cuFFT 145 us), 3072^2 176
-// (348), 6144^2 740 (1356), 8192^2 1691 (1961; there only two columns fit a CTA).
-// A line's trips through shared memory and the latency at 16 to 24 warps per SM
+// (348), 6144^2 740 (1356).  From 7168 on two columns fit a CTA instead of four and
+// one CTA's rows an SM, so that each gets all of the SM's threads: 7680^2 1610 us (with
+// cuFFT 2247), 8192^2 1722 (1978), 8000^2 1889 (1934), 7776^2 1948 (1858, the one
+// size at which cuFFT is faster); with the threads of the smaller sizes 1996, 2013, 2270
+// and 2496.  A line's trips through shared memory and the latency at 16 to 24 warps per SM
 // bound them.  Tried at 4096^2: radix 8 with every stage through shared memory
 // 322 us, twiddles gathered from one table of n roots 501 us; rows at two and four
-// CTAs per SM 260 and 253 us; two columns per CTA 358 us (radix 8).
+// CTAs per SM 260 and 253 us; two columns of 128 threads per CTA 358 us (radix 8).
 // Other sizes (a prime factor above 7, beyond 8192) stay with cuFFT.
 #include <float.h>
 #include <math.h>
@@ -49,8 +52,8 @@ namespace gb {
 namespace {
 
 constexpr int kMaxStages = 14;
-constexpr int kRowThreads = 256;
-constexpr int kColThreads = 128;  // per column
+constexpr int kRowRegs = 768;  // threads per SM that the rows' kernels leave registers for
+constexpr int kColThreads = 512;  // for all of a CTA's columns
 
 struct FftPlan {
   int n, stages;
@@ -320,7 +323,8 @@ __device__ __forceinline__ float correct(float a, float b) {
 
 // Image rows 2 b and 2 b + 1, corrected and signed, as the real and imaginary
 // part of one line; their half spectra are its even and odd parts.
-__global__ void __launch_bounds__(kRowThreads, 3)
+template <int T>
+__global__ void __launch_bounds__(T, kRowRegs / T)
     k_fft_rows_in(const float* __restrict__ x, const float* __restrict__ taper,
                   const __grid_constant__ FftPlan p, float2* __restrict__ g) {
   extern __shared__ __align__(16) float2 s[];
@@ -330,7 +334,7 @@ __global__ void __launch_bounds__(kRowThreads, 3)
   const float* x1 = x0 + n;
   const float t0 = taper ? taper[i] : 1.f, t1 = taper ? taper[i + 1] : 1.f;
   line_fft(
-      s, p, t, kRowThreads,
+      s, p, t, T,
       [&](int j) { return make_float3(__ldg(x0 + j), __ldg(x1 + j), taper ? __ldg(taper + j) : 1.f); },
       [&](int j, float3 q) {
         float a = q.x, b = q.y;
@@ -344,7 +348,7 @@ __global__ void __launch_bounds__(kRowThreads, 3)
       [&](int f, float2 a) { s2[at(f)] = a; });
   __syncthreads();
   float2* g0 = g + (int64_t)i * n;
-  for (int v = t; v <= n / 2; v += kRowThreads) {
+  for (int v = t; v <= n / 2; v += T) {
     const float2 a = s2[at(v)], b = s2[at(v ? n - v : 0)];
     g0[v] = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
     g0[n + v] = make_float2(0.5f * (a.y + b.y), 0.5f * (b.x - a.x));
@@ -353,14 +357,14 @@ __global__ void __launch_bounds__(kRowThreads, 3)
 
 // C columns v0 .. of the half spectrum, in place, and their mirror columns.
 template <int C>
-__global__ void __launch_bounds__(C* kColThreads, 1)
+__global__ void __launch_bounds__(kColThreads, 1)
     k_fft_cols_out(const __grid_constant__ FftPlan p, float2* __restrict__ g) {
   extern __shared__ __align__(16) float2 s[];
   const int n = p.n, h = n / 2;
   const int c = threadIdx.x % C, t = threadIdx.x / C, v = C * blockIdx.x + c;
   const int vl = min(v, h);  // the last CTA's spare columns transform a copy
   line_fft(
-      s + c * line(n), p, t, kColThreads, [&](int u) { return g[(int64_t)u * n + vl]; },
+      s + c * line(n), p, t, kColThreads / C, [&](int u) { return g[(int64_t)u * n + vl]; },
       [](int, float2 a) { return a; },
       [&](int u, float2 a) {
         if (v > h) return;
@@ -375,7 +379,7 @@ __global__ void __launch_bounds__(C* kColThreads, 1)
 // The Hermitian half of the grid's columns v0 .., transformed (exp(+2 pi i):
 // real and imaginary parts trade places on the way in and out) into w.
 template <int C>
-__global__ void __launch_bounds__(C* kColThreads, 1)
+__global__ void __launch_bounds__(kColThreads, 1)
     k_fft_cols_in(const float2* __restrict__ g, const __grid_constant__ FftPlan p,
                   float2* __restrict__ w) {
   extern __shared__ __align__(16) float2 s[];
@@ -383,7 +387,7 @@ __global__ void __launch_bounds__(C* kColThreads, 1)
   const int c = threadIdx.x % C, t = threadIdx.x / C, v = C * blockIdx.x + c;
   const int vl = min(v, h), vm = vl ? n - vl : 0;
   line_fft(
-      s + c * line(n), p, t, kColThreads,
+      s + c * line(n), p, t, kColThreads / C,
       [&](int u) {
         const float2 a = __ldg(g + (int64_t)u * n + vl);
         const float2 b = __ldg(g + (int64_t)(u ? n - u : 0) * n + vm);
@@ -402,7 +406,8 @@ constexpr int kOut = 4;  // pixels of a row that a thread takes together
 
 // Rows 2 b and 2 b + 1 of w, Hermitian along v, as one complex line: its
 // transform's real part is the first image row, its imaginary part the second.
-__global__ void __launch_bounds__(kRowThreads, 3)
+template <int T>
+__global__ void __launch_bounds__(T, kRowRegs / T)
     k_fft_rows_out(const float2* __restrict__ w, const float* __restrict__ taper,
                    const __grid_constant__ FftPlan p, float* __restrict__ x) {
   extern __shared__ __align__(16) float2 s[];
@@ -410,7 +415,7 @@ __global__ void __launch_bounds__(kRowThreads, 3)
   float2* s2 = s + line(n);
   const float2* w0 = w + (int64_t)i * n;
   line_fft(
-      s, p, t, kRowThreads,
+      s, p, t, T,
       [&](int v) {
         const int u = v <= h ? v : n - v;
         const float2 a = __ldg(w0 + u), b = __ldg(w0 + n + u);
@@ -427,18 +432,18 @@ __global__ void __launch_bounds__(kRowThreads, 3)
   __syncthreads();
   float* x0 = x + (int64_t)i * n;
   const float t0 = taper ? taper[i] : 1.f, t1 = taper ? taper[i + 1] : 1.f;
-  for (int j0 = t; j0 < n; j0 += kOut * kRowThreads) {
+  for (int j0 = t; j0 < n; j0 += kOut * T) {
     float2 a[kOut];
     float tj[kOut];
 #pragma unroll
     for (int k = 0; k < kOut; k++) {
-      const int j = min(j0 + k * kRowThreads, n - 1);
+      const int j = min(j0 + k * T, n - 1);
       a[k] = s2[at(j)];
       tj[k] = taper ? __ldg(taper + j) : 1.f;
     }
 #pragma unroll
     for (int k = 0; k < kOut; k++) {
-      const int j = j0 + k * kRowThreads;
+      const int j = j0 + k * T;
       const float sg = sign_of(j);
       const float u = sg * a[k].y, v = -sg * a[k].x;
       if (j < n) {
@@ -563,6 +568,9 @@ constexpr size_t kFftSmem = 224 * 1024;
 // Columns per CTA: four where they fit (a row of them is one 32-byte sector).
 int columns(int n) { return line_bytes(n, 4) <= kFftSmem ? 4 : 2; }
 
+// Threads for a pair of rows: 256, and 512 where two CTAs' lines do not fit an SM.
+int row_threads(int n) { return line_bytes(n, 4) <= kFftSmem ? 256 : 512; }
+
 // The kernels' shared-memory limit, set once per device.
 int set_limits() {
   static std::mutex mu;
@@ -571,7 +579,8 @@ int set_limits() {
   GB_CUDA_TRY(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(mu);
   if (dev >= 0 && dev < 64 && done[dev]) return GB_OK;
-  for (const void* fn : {(const void*)k_fft_rows_in, (const void*)k_fft_rows_out,
+  for (const void* fn : {(const void*)k_fft_rows_in<256>, (const void*)k_fft_rows_in<512>,
+                         (const void*)k_fft_rows_out<256>, (const void*)k_fft_rows_out<512>,
                          (const void*)k_fft_cols_out<4>, (const void*)k_fft_cols_out<2>,
                          (const void*)k_fft_cols_in<4>, (const void*)k_fft_cols_in<2>})
     GB_CUDA_TRY(
@@ -593,11 +602,14 @@ int fft_image_to_grid(const float* x, const float* taper, int n, float2* g, cuda
   if (rc) return rc;
   const int C = columns(n), groups = (n / 2 + C) / C;
   if ((rc = set_limits())) return rc;
-  k_fft_rows_in<<<n / 2, kRowThreads, line_bytes(n, 2), s>>>(x, taper, p, g);
-  if (C == 4)
-    k_fft_cols_out<4><<<groups, 4 * kColThreads, line_bytes(n, 4), s>>>(p, g);
+  if (row_threads(n) == 256)
+    k_fft_rows_in<256><<<n / 2, 256, line_bytes(n, 2), s>>>(x, taper, p, g);
   else
-    k_fft_cols_out<2><<<groups, 2 * kColThreads, line_bytes(n, 2), s>>>(p, g);
+    k_fft_rows_in<512><<<n / 2, 512, line_bytes(n, 2), s>>>(x, taper, p, g);
+  if (C == 4)
+    k_fft_cols_out<4><<<groups, kColThreads, line_bytes(n, 4), s>>>(p, g);
+  else
+    k_fft_cols_out<2><<<groups, kColThreads, line_bytes(n, 2), s>>>(p, g);
   GB_CUDA_TRY(cudaGetLastError());
   return GB_OK;
 }
@@ -610,10 +622,13 @@ int fft_grid_to_image(const float2* g, const float* taper, int n, float2* w, flo
   const int C = columns(n), groups = (n / 2 + C) / C;
   if ((rc = set_limits())) return rc;
   if (C == 4)
-    k_fft_cols_in<4><<<groups, 4 * kColThreads, line_bytes(n, 4), s>>>(g, p, w);
+    k_fft_cols_in<4><<<groups, kColThreads, line_bytes(n, 4), s>>>(g, p, w);
   else
-    k_fft_cols_in<2><<<groups, 2 * kColThreads, line_bytes(n, 2), s>>>(g, p, w);
-  k_fft_rows_out<<<n / 2, kRowThreads, line_bytes(n, 2), s>>>(w, taper, p, x);
+    k_fft_cols_in<2><<<groups, kColThreads, line_bytes(n, 2), s>>>(g, p, w);
+  if (row_threads(n) == 256)
+    k_fft_rows_out<256><<<n / 2, 256, line_bytes(n, 2), s>>>(w, taper, p, x);
+  else
+    k_fft_rows_out<512><<<n / 2, 512, line_bytes(n, 2), s>>>(w, taper, p, x);
   GB_CUDA_TRY(cudaGetLastError());
   return GB_OK;
 }
