@@ -60,7 +60,7 @@ constexpr int kMaxItems = kMaxBins + 4096;  // bins are cut: one item each and 4
 
 // byte layout of the scratch array (the cursors follow the histogram's bins in
 // use, so that one memset clears counters, histogram and cursors)
-constexpr size_t kOffCounters = 0;  // int32[16]: pieces, items, bundles, queue
+constexpr size_t kOffCounters = 0;  // int32[16]: pieces, bundles, queue
 constexpr size_t kOffHist = 256;
 constexpr size_t kOffOffs = align256(kOffHist + 8 * (size_t)kMaxBins);
 constexpr size_t kOffCells = align256(kOffOffs + 4 * ((size_t)kMaxBins + 1));
@@ -71,7 +71,8 @@ constexpr size_t kScratchBytes = align256(kOffBundles + sizeof(Bundle) * (size_t
 static_assert(kScratchBytes <= (size_t)GB_NOALLOC_SCRATCH_BYTES,
               "scratch layout exceeds the documented size");
 
-enum { kCntPieces = 0, kCntItems = 1, kCntBundles = 2, kCntQueue = 3 };
+// (the pieces are for the bounds-checked build)
+enum { kCntPieces = 0, kCntBundles = 1, kCntQueue = 2 };
 
 struct NaPlanes {  // by value: a kernel argument
   PlaneInfo p[kMaxPlanes];
@@ -179,7 +180,6 @@ __global__ void __launch_bounds__(1024) k_na_tables(const int32_t* __restrict__ 
   if (tid == 1023) {
     offs[nkeys] = rpre;
     counters[kCntPieces] = rpre;
-    counters[kCntItems] = ipre;
     cls_first[nc.n] = ipre;
   }
   __syncthreads();
@@ -387,7 +387,10 @@ extern "C" int gb_grid_f32_noalloc(const gb_geometry* geo, int64_t n_vis, const 
   }
   nc.ntiles = (int32_t)ntiles;
   // items of 32 pieces or more, four per SM for larger calls, and never more than
-  // 4096 beyond one per bin
+  // 4096 beyond one per bin.  (With the caller's zeroing, 4,560 visibilities of 96
+  // stations: items of 8 / 16 / 32 / 64 / 128 pieces 65 / 65 / 67 / 69 / 73 us, 18,240: 77 / 76 /
+  // 77 / 82 / 89.  130,560 of 256 stations: two / four / eight / sixteen per SM 222 / 185 / 171
+  // / 179, 79,600 of 200: 161 / 140 / 134 / 142.)
   const int64_t pieces = n_vis * kmax * kmax;
   nc.cut = (int32_t)std::max<int64_t>({32, (pieces + 4095) / 4096, pieces / (4 * sm_count())});
 
@@ -435,5 +438,5 @@ extern "C" int gb_grid_f32_noalloc(const gb_geometry* geo, int64_t n_vis, const 
   return launch_grid_tiled_tables(bundles, counters + kCntBundles, (int)most, items, recs,
                                   counters + kCntQueue, cls, nwidth, NT, T, geo->ext_x, geo->ext_y,
                                   geo->pitch, smem, d_vis, d_gcf, d_grid,
-                                  TiledBounds{kMaxPieces, gcf_len, n_vis}, s);
+                                  TiledBounds{kMaxPieces, gcf_len, n_vis, counters + kCntPieces}, s);
 }

@@ -245,6 +245,7 @@ int plan_create(const gb_geometry* geo, int64_t n_vis, const double* d_uvw, int6
 // Array sizes behind a launch's pointers (used by the bounds-checked build).
 struct TiledBounds {
   int64_t n_recs, gcf_len, n_vis;
+  const int32_t* n_recs_dev = nullptr;  // the number of records where only the device has it
 };
 int launch_grid_tiled_tables(const Bundle* bundles, const int32_t* n_bundles, int max_bundles,
                              const Item* items, const Rec* recs, int32_t* queue,

@@ -51,6 +51,7 @@ struct TiledArgs {
   int32_t T;
 #ifdef GB_CHECKED
   int64_t n_recs;   // records in `recs`
+  const int32_t* n_recs_dev;  // where that is on the device, or NULL
   int64_t gcf_len;  // complex elements in the GCF array
 #endif
 };
@@ -70,6 +71,9 @@ __device__ __forceinline__ int64_t gb_checked_index(int64_t i, int64_t lim) {
   return i;
 }
 #define GB_IDX(i, lim) gb_checked_index((int64_t)(i), (int64_t)(lim))
+__device__ __forceinline__ int64_t recs_len(const TiledArgs& a) {
+  return a.n_recs_dev ? *a.n_recs_dev : a.n_recs;
+}
 #else
 #define GB_IDX(i, lim) (i)
 #endif
@@ -291,7 +295,7 @@ __device__ __forceinline__ void grid_item(const TiledArgs& a, const Item& it, in
     const int nb = min(L, end - base);
     group_sync(bar, L, whole);  // zeroing done / previous batch consumed
     if (lt < nb) {
-      const Rec r = a.recs[GB_IDX(base + lt, a.n_recs)];
+      const Rec r = a.recs[GB_IDX(base + lt, recs_len(a))];
       GridRec d;
       d.gcf = (int32_t)r.gcf;
       d.q0 = r.yl * As + r.xl;
@@ -555,7 +559,7 @@ __device__ __forceinline__ void degrid_item(const TiledArgs& a, const Item& it, 
     const int nb = min(L, end - base);
     group_sync(bar, L, whole);  // previous batch consumed
     if (lt < nb) {
-      const Rec r = a.recs[GB_IDX(base + lt, a.n_recs)];
+      const Rec r = a.recs[GB_IDX(base + lt, recs_len(a))];
       DegridRec d;
       d.gcf = (int32_t)r.gcf;
       d.pitch = r.sm1 + 1;
@@ -855,6 +859,7 @@ int tiled_ctas_per_sm(const gb_plan* P, bool grid, int stage) {
 static void set_bounds(TiledArgs& a, const TiledBounds& b) {
 #ifdef GB_CHECKED
   a.n_recs = b.n_recs;
+  a.n_recs_dev = b.n_recs_dev;
   a.gcf_len = b.gcf_len;
 #else
   (void)a;
