@@ -11,14 +11,15 @@
 // lazy: the image is cut into 32 x 16 tiles, dealt out to the warps; a tile keeps
 // the maximum it had when it was last brought up to date and an upper bound of
 // what the components since then can have made of it (|s| times the largest
-// |psf| over the part that covers the tile, from a table of block maxima,
-// rounded up; only the PSF's window that can lie on the image).  After a component the next peak is at least what is left at the
-// old one, so only tiles whose bound reaches that are brought up to date: a few
-// around the bright sources instead of the whole image.  The others take their
-// pending components later, several per pass over their pixels (when a tile's
-// bound rises, when the list of components is full, at the end), each pixel in
-// the components' order, with unfused arithmetic (__fmul_rn / __fsub_rn), so
-// every pixel and every peak is what a numpy float32 loop computes, bit for bit.
+// |psf| over the part that covers the tile, rounded up, from a table of block
+// maxima of the PSF's window that can lie on the image).  After a component the
+// next peak is at least what is left at the old one, so only tiles whose bound
+// reaches that are brought up to date: a few around the bright sources instead of
+// the whole image.  The others take their pending components later, several per
+// pass over their pixels (when a tile's bound rises, when the list of components is
+// full, at the end), each pixel in the components' order, with unfused arithmetic
+// (__fmul_rn / __fsub_rn), so every pixel and every peak is what a numpy float32
+// loop computes, bit for bit.
 // Per iteration each CTA publishes its best candidate and reads all the others'.
 // Reference form, kern_hogbom_model / kern_hogbom_residual: the reference's
 // Halide CLEAN (MS6/kernel/cpu/gridding/hogbom.cpp:10-109) restated on the GPU

@@ -718,8 +718,9 @@ __device__ __forceinline__ void degrid_item(const TiledArgs& a, const Item& it, 
       // parts and the upper half the imaginary ones; the rest then reduces one
       // value a lane, log2(SW) shuffles a record instead of twice that.  A
       // shuffle takes two cycles of the L1 data path, which bounds this kernel
-      // (84 to 87 % busy), and with two values they were 14 % of it (32 w-planes,
-      // 4.18e6 visibilities: 1168 us before, 1150 now).  Same sums, same order.
+      // (84 to 87 % busy), and with two values they were 14 % of it.  (32 w-planes,
+      // 4.18e6 visibilities: 1.00x to 1.02x in paired runs, about what runs differ.)
+      // Same sums, same order.
       constexpr int H = SW / 2;
       const bool upper = (sl & H) != 0;
       float sum = upper ? ai : ar;
