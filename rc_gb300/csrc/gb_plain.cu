@@ -522,17 +522,23 @@ static int single_degrid_dims(int64_t n, int S, int* blocks, int* pw) {
 // visibilities per warp 2826 and 1355, with 64 / 320 warps per SM 2786 / 2336 and
 // 1259 / 1105.  But the indexing, one visibility per lane, is repeated per warp, and
 // small footprints (the largest support says it) are too little work for that:
-//   supports to 8: at least 8 per warp, and 32 (grid) or 64 (degrid) warps per SM.
+//   supports to 8: 8 per warp or more as long as an SM has eight warps (2,000 and fewer: one
+//     per warp, 22 and 45 us, 26 and 50 with eight), and 32 (grid) or 64 (degrid) per SM.
 //     129,024 of support 8: at 320 per SM 150 and 198 us, at 64 98 and 149; 65,000 of
 //     support 4: at 320 85 and 166, at 64 47 and 115, at 32 42 and 111;
-//   supports to 24: 64 and 128.  65,000 of support 16: at 320 194 and 180 us, at 128 172
-//     and 160, at 64 160 and 155; 520,000: 1061, 1022, 1053 and 527, 527, 543.
+//   supports to 24: 4 per warp or more likewise, and 80 (grid) or 128 (degrid).  Grid at 320 /
+//     128 / 96 / 80 / 64: 65,000 of support 10 132, 109, 102, 97, 96 us, of support 20 271,
+//     253, 244, 236, 242; 260,000 of support 16 578, 554, 531, 533, 522; a core-heavy
+//     211,854 of 8 to 26 441, 350, 359, 384, 409.  Degrid at 320 / 128 / 64: 65,000 of
+//     support 16 180, 160, 155; 520,000 527, 527, 543.
 //   Supports to 32, 65,000: at 320 557 and 290, at 64 541 and 289 us; to 48: 1161 and
 //     498, 1173 and 519.
 static int plain_grid_dims(int64_t n, int max_support, bool grid, int* blocks, int* pw) {
-  const int per_sm = max_support <= 8 ? (grid ? 32 : 64) : max_support <= 24 ? (grid ? 64 : 128) : 320;
+  const int per_sm = max_support <= 8 ? (grid ? 32 : 64) : max_support <= 24 ? (grid ? 80 : 128) : 320;
+  const int64_t least = std::clamp<int64_t>(n / (sm_count() * 8), 1,
+                                            max_support <= 8 ? 8 : max_support <= 24 ? 4 : 1);
   const int64_t target = (int64_t)sm_count() * per_sm;
-  *pw = (int)std::clamp<int64_t>((n + target - 1) / target, max_support <= 8 ? 8 : 1, 32);
+  *pw = (int)std::clamp<int64_t>((n + target - 1) / target, least, 32);
   const int64_t warps = (n + *pw - 1) / *pw;
   *blocks = (int)std::clamp<int64_t>((warps + 7) / 8, 1, 1 << 30);
   return 256;

@@ -49,7 +49,7 @@ def test_blocks_spread_over_the_order(blocks, extra):
     _check(64 * blocks + extra, [3, 8], 0.5)  # eight visibilities a warp, eight warps a block
 
 
-@pytest.mark.parametrize("supports,per_sm", [([1, 2, 4], 32), ([1, 2, 4], 64), ([1, 9], 64), ([1, 9], 128),
+@pytest.mark.parametrize("supports,per_sm", [([1, 2, 4], 32), ([1, 2, 4], 64), ([1, 9], 80), ([1, 9], 128),
                                              ([1, 25], 320)])
 @pytest.mark.parametrize("share,extra", [(1, 0), (1, 1), (8, 1), (31, 1), (32, 0), (32, 1)])
 def test_shares(supports, per_sm, share, extra):
