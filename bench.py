@@ -456,7 +456,7 @@ def device_pair(ob, args, dev, flush, clock_index=0, steps=None, fp64_reps=None)
     G = ob.grid_size
     tp = Gm.pswf_taper(ob.max_support)
     gen = []
-    for _ in range(2):  # the first call creates cuFFT plans and loads the library
+    for _ in range(2):  # the first call loads the library
         t0 = time.perf_counter()
         g64, g32, offs = Gm.generate(ob.w_planes, ob.supports, ob.max_support, ob.scale / 2,
                                      taper=tp, device=dev)

@@ -287,12 +287,13 @@ int gb_degrid_backward_f64(gb_plan *plan, const double *d_gcf, const double *d_p
 /* On-GPU w-kernel generation (MS4/kernel/cpu/gcf/GCF.cpp semantics): for
  * each plane p, the FP64 phase screen exp(-2 pi i w_p (1 - sqrt(1-l^2-m^2)))
  * times taper(l) taper(m) on a max_support^2 patch (l, m = k * t2 /
- * (max_support/2)), centred in an (8 max_support)^2 arena, centred inverse
- * FFT (cuFFT, FP64), per-phase normalisation by the sum of real parts, and
- * extraction of the centred S_p x S_p taps per phase.  Writes complex128
+ * (max_support/2)), as centred in an (8 max_support)^2 arena, its centred inverse
+ * FFT in FP64, per-phase normalisation by the sum of real parts, and the centred S_p
+ * x S_p taps per phase.  (Transforms pruned to the patch and the taps where
+ * max_support has no prime factor above 7, cuFFT of the whole arena otherwise.)  Writes complex128
  * (d_gcf64, may be NULL) and complex64 (d_gcf32, may be NULL) GCF arrays laid
  * out by gcf_offsets.  d_taper: device, max_support doubles, or NULL for none.
- * Allocates its FFT workspace per call. */
+ * Allocates its workspace per call. */
 int gb_gcf_generate(int32_t n_planes, const double *w_planes, const int32_t *supports,
                     const int64_t *gcf_offsets, int32_t max_support, double t2,
                     const double *d_taper, double *d_gcf64, float *d_gcf32, void *stream);

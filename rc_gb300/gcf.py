@@ -7,7 +7,7 @@
 * pswf(): prolate spheroidal wave function (order 0) via scipy.special.pro_ang1;
 * pswf_uv_gcf(): an oversampled uv-domain PSWF GCF for the no-w-term case;
 * generate(): on-GPU w-kernel generation through gb_gcf_generate (FP64 phase
-  screens + cuFFT), returning complex128 and/or complex64 device tensors.
+  screens and their transforms), returning complex128 and/or complex64 device tensors.
 """
 from __future__ import annotations
 
