@@ -226,63 +226,35 @@ struct ItemRule {
   double pieces;  // items wanted per unit of total cost: bundles per CTA x CTAs
 };
 
-// The items of each (class, tile): counted (per class, tile-fastest), or with
-// `items` written from first[] on.  An item is closed when its cost reaches the
-// larger of four times its fixed cost and an even share of all the work.
-// A thread to a (class, tile).  Most are empty or give an item or two, but a core-heavy
-// array puts much of its work into a few tiles, each of thousands of items: those of
-// one period are alike, so they are counted by a division and written by the whole warp.
-// A plan of 1e6 visibilities of support 8, all in one tile: 0.71 ms, with a thread
-// cutting its items one by one 4.7 ms (on host threads 2.5 ms); 8e6: 1.45 ms, 4.9
-// and 11.7; 1e6 of a core-heavy array on 256^2: 0.81 ms, 2.96 and 1.92.
-__global__ void __launch_bounds__(128)
-    k_plan_items(const __grid_constant__ ItemRule R, int64_t ntiles, int32_t ntx,
-                 const int32_t* __restrict__ offs, PlanCounts* __restrict__ cnt,
-                 int32_t* __restrict__ count, const int32_t* __restrict__ first,
-                 Item* __restrict__ items, float* __restrict__ costs) {
-  __shared__ float s_tau;
-  __shared__ bool s_over;
-  if (threadIdx.x == 0) {
-    double total = 0;
-    for (int r = 0; r < R.nper; r++) total += (double)cnt->rank[r] * R.per_cta[r];
-    s_tau = (float)(total / R.pieces);
-    s_over = cnt->recs >= (unsigned long long)INT32_MAX;  // refused by the host: offs wrapped
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int c = min((int)(e / ntiles), R.nclass - 1);
-  const int64_t tile = e % ntiles;
-  const bool live = e < ntiles * R.nclass;
-  bool used = false, any = false;
+// Writes the items (where `items` is given, from index `at` on) of one tile's records
+// of class c; returns how many.  An item is closed when its cost reaches cmax.  By one
+// thread; or by a warp, all of whose lanes walk the same way: items of one rank alone are
+// alike from the first record of one on, so the warp counts them by a division and
+// writes them side by side.
+template <bool kWarp>
+__device__ __forceinline__ int cut_items(const ItemRule& R, const int32_t* __restrict__ offs,
+                                         int64_t tile, int ntx, int c, float cmax, int64_t at,
+                                         Item* __restrict__ items, float* __restrict__ costs) {
   const int64_t k0 = tile * R.nper;
-  int32_t start = 0;
-  if (live && !s_over) {
-    start = offs[k0 + R.lo[c]];
-    any = start != offs[k0 + R.hi[c]];
-    used = c == 0 && offs[k0 + R.nper] != offs[k0];
-  }
-  const float fixed = R.fixed[c], cmax = fmaxf(4.f * fixed, s_tau);
-  int64_t at = items && any ? first[e] : 0;
+  const int lane = threadIdx.x & 31;
+  const float fixed = R.fixed[c];
   float cost = fixed;
-  int32_t in_item = 0, n = 0;
+  int32_t start = offs[k0 + R.lo[c]], in_item = 0;
   int64_t top_taps = 0;
-  int top = -1, pmax = 0;
-  auto write = [&](int64_t to, int64_t tile_, int c_, int32_t start_, int32_t count_, int pmax_, int top_,
-                   float cost_) {
+  int n = 0, top = -1, pmax = 0;
+  auto write = [&](int64_t i, int32_t first, int32_t records, int p, int rank, float item_cost) {
     Item it;
-    it.start = start_;
-    it.count = count_;
-    it.tile_x = (int16_t)(tile_ % ntx);
-    it.tile_y = (int16_t)(tile_ / ntx);
-    it.pmax = (int16_t)pmax_;
-    it.cls = item_cls_with_residue((int16_t)c_, R.residue[top_]);
-    items[to] = it;
-    costs[to] = cost_;
+    it.start = first;
+    it.count = records;
+    it.tile_x = (int16_t)(tile % ntx);
+    it.tile_y = (int16_t)(tile / ntx);
+    it.pmax = (int16_t)p;
+    it.cls = item_cls_with_residue((int16_t)c, R.residue[rank]);
+    items[i] = it;
+    costs[i] = item_cost;
   };
   auto close = [&]() {
-    if (items) write(at, tile, c, start, in_item, pmax, top, cost);
-    at++;
+    if (items && (!kWarp || lane == 0)) write(at + n, start, in_item, pmax, top, cost);
     n++;
     start += in_item;
     in_item = 0;
@@ -290,66 +262,107 @@ __global__ void __launch_bounds__(128)
     top_taps = 0;
     pmax = 0;
   };
-  // as many records of rank r as the open item has room for
-  auto step = [&](int r, int32_t& pos, int32_t end) {
-    const float rc = R.rec[r], room = fminf((cmax - cost) * (1.f / rc), 2e9f);
-    const int32_t take = min(max((int32_t)room, 1), end - pos);
-    const int64_t t = (int64_t)take * R.period[r] * R.period[r];
-    if (t > top_taps) {  // the stage stride goes by the largest run
-      top_taps = t;
-      top = r;
-    }
-    pmax = R.period[r];
-    in_item += take;
-    cost += (float)take * rc;
-    pos += take;
-    if (cost >= cmax) close();
-  };
-  const int r0 = __reduce_min_sync(0xffffffffu, any ? R.lo[c] : R.nper);
-  const int r1 = __reduce_max_sync(0xffffffffu, any ? R.hi[c] : 0);
-  for (int r = r0; r < r1; r++) {
-    int32_t pos = 0, end = 0, whole = 0, per = 0;
-    float per_cost = fixed;
-    if (any && r >= R.lo[c] && r < R.hi[c]) {
-      pos = offs[k0 + r];
-      end = offs[k0 + r + 1];
-      while (in_item && pos < end) step(r, pos, end);
-      if (pos < end) {  // the records of an item of this rank alone, step by step
-        const float rc = R.rec[r];
-        while (per_cost < cmax && per < end - pos) {
-          const float room = fminf((cmax - per_cost) * (1.f / rc), 2e9f);
-          const int32_t take = min(max((int32_t)room, 1), end - pos - per);
-          per_cost += (float)take * rc;
-          per += take;
+  for (int r = R.lo[c]; r < R.hi[c]; r++) {
+    int32_t pos = offs[k0 + r];
+    const int32_t end = offs[k0 + r + 1];
+    const float rc = R.rec[r], per = 1.f / rc;
+    int32_t alike0 = -1;  // where the last item that began with this rank did
+    while (pos < end) {
+      if (kWarp && !in_item) {
+        if (alike0 >= 0) {  // the one before is of this rank alone: so are the next m
+          const int32_t recs = pos - alike0, m = (end - pos) / recs;
+          float item_cost = fixed;
+          for (int32_t k = 0; k < recs && m > 0;) {  // its cost, step by step
+            const int32_t take = min(max((int32_t)fminf((cmax - item_cost) * per, 2e9f), 1), recs - k);
+            item_cost += (float)take * rc;
+            k += take;
+          }
+          if (items)
+            for (int i = lane; i < m; i += 32)
+              write(at + n + i, pos + i * recs, recs, R.period[r], r, item_cost);
+          n += m;
+          pos += m * recs;
+          start = pos;
+          alike0 = -1;
+          if (m > 0) continue;
         }
-        if (per_cost >= cmax) whole = (end - pos) / per;
+        alike0 = pos;
       }
-    }
-    if (items) {
-      for (unsigned many = __ballot_sync(0xffffffffu, whole >= 32); many; many &= many - 1) {
-        const int src = __ffs(many) - 1;
-        const int64_t to = __shfl_sync(0xffffffffu, at, src), tl = __shfl_sync(0xffffffffu, tile, src);
-        const int cl = __shfl_sync(0xffffffffu, c, src), m = __shfl_sync(0xffffffffu, whole, src);
-        const int32_t p = __shfl_sync(0xffffffffu, per, src), s0 = __shfl_sync(0xffffffffu, pos, src);
-        const float pc = __shfl_sync(0xffffffffu, per_cost, src);
-        for (int i = lane; i < m; i += 32) write(to + i, tl, cl, s0 + i * p, p, R.period[r], r, pc);
+      const float room = fminf((cmax - cost) * per, 2e9f);
+      const int32_t take = min(max((int32_t)room, 1), end - pos);
+      const int64_t t = (int64_t)take * R.period[r] * R.period[r];
+      if (t > top_taps) {  // the stage stride goes by the largest run
+        top_taps = t;
+        top = r;
       }
-      if (whole < 32)
-        for (int i = 0; i < whole; i++) write(at + i, tile, c, pos + i * per, per, R.period[r], r, per_cost);
+      pmax = R.period[r];
+      in_item += take;
+      cost += (float)take * rc;
+      pos += take;
+      if (cost >= cmax) close();
     }
-    if (whole) {
-      at += whole;
-      n += whole;
-      pos += whole * per;
-      start = pos;
-    }
-    while (pos < end) step(r, pos, end);
   }
   if (in_item) close();
-  if (!items) {
-    if (live) count[e] = n;
-    const int used_here = __syncthreads_count(used);
-    if (threadIdx.x == 0 && used_here) atomicAdd(&cnt->tiles, (unsigned long long)used_here);
+  return n;
+}
+
+constexpr int kItemThreads = 128;
+constexpr float kWarpItems = 128.f;  // at least, for a warp to cut them
+
+// The items of each (class, tile): counted (per class, tile-fastest), or with
+// `items` written from first[] on.  cmax: the larger of four times an item's fixed
+// cost and an even share of all the work.
+// A thread to a (class, tile): most are empty or give an item or a few.  But a
+// core-heavy array puts much of its work into a few tiles, each of hundreds or
+// thousands of items: those are left for the block's warps.  A plan of 1e6 visibilities
+// of support 8, all in one tile: 0.66 ms, with a thread to each tile 4.6 ms (on host
+// threads 2.3 ms); 8e6: 1.4 ms, 4.8 and 11.6; 1e6 of a core-heavy array on 256^2: 0.79 ms,
+// 2.9 and 1.8.  Every lane in step over the ranks of all tiles took 10 us longer where
+// the tiles are sparse (39 -> 49 us on 16384^2, 31 ranks).
+__global__ void __launch_bounds__(kItemThreads)
+    k_plan_items(const __grid_constant__ ItemRule R, int64_t ntiles, int32_t ntx,
+                 const int32_t* __restrict__ offs, PlanCounts* __restrict__ cnt,
+                 int32_t* __restrict__ count, const int32_t* __restrict__ first,
+                 Item* __restrict__ items, float* __restrict__ costs) {
+  __shared__ float s_tau;
+  __shared__ bool s_over;
+  __shared__ int s_dense;
+  __shared__ int32_t s_entry[kItemThreads];
+  if (threadIdx.x == 0) {
+    double total = 0;
+    for (int r = 0; r < R.nper; r++) total += (double)cnt->rank[r] * R.per_cta[r];
+    s_tau = (float)(total / R.pieces);
+    s_over = cnt->recs >= (unsigned long long)INT32_MAX;  // refused by the host: offs wrapped
+    s_dense = 0;
+  }
+  __syncthreads();
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int c = (int)(e / ntiles);
+  bool used = false;
+  if (c < R.nclass) {
+    const int64_t tile = e - c * ntiles, k0 = tile * R.nper;
+    const int32_t b0 = offs[k0 + R.lo[c]], b1 = offs[k0 + R.hi[c]];
+    used = c == 0 && offs[k0 + R.nper] != offs[k0];
+    int n = 0;
+    if (b1 != b0 && !s_over) {
+      const float cmax = fmaxf(4.f * R.fixed[c], s_tau);
+      if ((float)(b1 - b0) * R.rec[R.lo[c]] >= kWarpItems * (cmax - R.fixed[c]))
+        s_entry[atomicAdd(&s_dense, 1)] = threadIdx.x;
+      else
+        n = cut_items<false>(R, offs, tile, ntx, c, cmax, items ? first[e] : 0, items, costs);
+    }
+    if (!items) count[e] = n;
+  }
+  // (the dense ones' counts after the zeros above)
+  const int used_here = __syncthreads_count(used);
+  if (!items && threadIdx.x == 0 && used_here)
+    atomicAdd(&cnt->tiles, (unsigned long long)used_here);
+  for (int k = threadIdx.x >> 5; k < s_dense; k += kItemThreads / 32) {
+    const int64_t d = blockIdx.x * (int64_t)blockDim.x + s_entry[k];
+    const int dc = (int)(d / ntiles);
+    const int n = cut_items<true>(R, offs, d - dc * ntiles, ntx, dc, fmaxf(4.f * R.fixed[dc], s_tau),
+                                  items ? first[d] : 0, items, costs);
+    if (!items && (threadIdx.x & 31) == 0) count[d] = n;
   }
 }
 
@@ -819,8 +832,8 @@ static int build_plan(gb_plan* P, const gb_geometry* geo, int64_t n_vis, const d
     }
   }
   R.pieces = (double)P->bpc * std::max(1, sm_count() * std::max(1, P->ctas_per_sm_grid));
-  const int iblocks = (int)((nci + 127) / 128);
-  k_plan_items<<<iblocks, 128, 0, s>>>(R, ntiles, P->ntx, d_offs, d_cnt, d_icount, nullptr, nullptr,
+  const int iblocks = (int)((nci + kItemThreads - 1) / kItemThreads);
+  k_plan_items<<<iblocks, kItemThreads, 0, s>>>(R, ntiles, P->ntx, d_offs, d_cnt, d_icount, nullptr, nullptr,
                                        nullptr);
   GB_CUDA_TRY(cudaGetLastError());
   if ((rc = scan_keys(d_icount, nci, d_ifirst, d_sums, s))) return rc;
@@ -856,7 +869,7 @@ static int build_plan(gb_plan* P, const gb_geometry* geo, int64_t n_vis, const d
     k_plan_fill<<<blocks_for(n_vis, 256), 256, 0, s>>>(D, P->d_planes, d_cells, P->T, P->ntx, nper,
                                                        d_offs, d_hist, P->d_recs, d_offs + nkeys,
                                                        d_vhist, P->d_order);
-  k_plan_items<<<iblocks, 128, 0, s>>>(R, ntiles, P->ntx, d_offs, d_cnt, nullptr, d_ifirst,
+  k_plan_items<<<iblocks, kItemThreads, 0, s>>>(R, ntiles, P->ntx, d_offs, d_cnt, nullptr, d_ifirst,
                                        P->d_raw_items, P->d_raw_cost);
   GB_CUDA_TRY(cudaGetLastError());
   // a batch member's items go into the batch's own tables instead

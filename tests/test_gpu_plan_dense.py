@@ -1,5 +1,5 @@
 """The plan's work items where one tile holds most of the work: counts at and around
-whole items and at the number of them from which a warp writes them together, whole
+whole items and at the number of them from which a warp takes them together, whole
 items between rests of other periods, and the time a plan takes."""
 import time
 
@@ -38,7 +38,7 @@ def _sums(p, supports):
 PER = 48
 
 
-@pytest.mark.parametrize("items", [1, 2, 31, 32, 33, 64, 200])
+@pytest.mark.parametrize("items", [1, 2, 33, 95, 96, 97, 127, 128, 129, 130, 300])
 @pytest.mark.parametrize("extra", [-1, 0, 1])
 def test_items_of_one_period(items, extra):
     n = PER * items + extra
