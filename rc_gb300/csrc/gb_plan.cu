@@ -307,7 +307,10 @@ __device__ __forceinline__ int cut_items(const ItemRule& R, const int32_t* __res
 }
 
 constexpr int kItemThreads = 128;
-constexpr float kWarpItems = 128.f;  // at least, for a warp to cut them
+// Items from which a warp cuts them (counting and writing, us): from 128 / 64 / 32 / 16 a
+// core-heavy 1e6 of 29 planes on 1024^2 31 and 63 / 21 and 36 / 21 and 35 / 26 and 38, 1e5
+// of 31 planes on 256^2 37 and 76 / 42 and 75 / 58 and 90 / 69 and 105.
+constexpr float kWarpItems = 64.f;
 
 // The items of each (class, tile): counted (per class, tile-fastest), or with
 // `items` written from first[] on.  cmax: the larger of four times an item's fixed

@@ -38,7 +38,7 @@ def _sums(p, supports):
 PER = 48
 
 
-@pytest.mark.parametrize("items", [1, 2, 33, 95, 96, 97, 127, 128, 129, 130, 300])
+@pytest.mark.parametrize("items", [1, 2, 33, 63, 64, 65, 66, 127, 128, 129, 300])
 @pytest.mark.parametrize("extra", [-1, 0, 1])
 def test_items_of_one_period(items, extra):
     n = PER * items + extra
